@@ -681,6 +681,24 @@ struct C2PCount {
     unsigned newton = 0, bisect = 0, hydro_fallback = 0;
 };
 
+// The reference's fixed point p <- p - f(p), f = E + p - rho h W^2 (srhd_core.py:
+// 62-131), at most 60 steps from p0 = (gamma - 1)(E - D) clamped to
+// [1e-12, P_MAX]; a start that does not converge ends at p0 again.
+//
+// With W >= 1 and rho = D / W above its floor, rho h W^2 = D W + g p W^2 with
+// g = gamma / (gamma - 1), and E - D <= p0 / (gamma - 1) unless p0 was clamped
+// to P_MAX, so for every p >= p0
+//   -f(p) >= D (W - 1) + g p (W^2 - 1) + (p - p0) / (gamma - 1).
+// A first step upwards that is not yet within the tolerance is therefore
+// followed by steps upwards only, none of them smaller (gamma < 2): the
+// iteration runs away from its root to P_MAX, never converges, and the result
+// is p0.  (From a p0 clamped to P_MAX such a step returns to P_MAX, 60 times.)
+// That is what happens in every cell that moves faster than |v| ~ 1e-6, since
+// f(p0) is then negative beyond the tolerance; the other steps would be spent to
+// reach a value that is dropped, so the loop ends after the first.  This solve was
+// most of the float64 updates' time: 60 dependent steps of a square root and
+// four divisions (SRHD update of 134^3 cells 833 us with them, 197 us without;
+// RMHD, whose Newton start it is, 1213 and 599 us).
 AHD void s_c2p(const Phys<double>& P, const double* U, double* q) {
     const double gamma = P.srhd_gamma, SM = 1e-12;
     double D = U[0], Sx = U[1], Sy = U[2], Sz = U[3], tau = U[4];
@@ -706,6 +724,9 @@ AHD void s_c2p(const Phys<double>& P, const double* U, double* q) {
         if (pn < SM) pn = SM;
         if (pn > P.p_max) pn = P.p_max;
         if (fabs(dp) < 1e-12 * rmax(1.0, pn)) { p = pn; ok = true; break; }
+        // runs away (see above); D > 2e-12 W keeps rho off its floor for this
+        // and every larger p (W falls with p)
+        if (it == 0 && dp > 0.0 && D > 2.0 * SM * W && gamma > 1.0 && gamma < 2.0) break;
         p = pn;
     }
     if (!ok) {
