@@ -1,0 +1,298 @@
+// face64.cu -- the float64 face passes of the split stages and right-hand
+// sides.
+//
+// Reconstruction is cell-centred: both face values of a cell come from one
+// evaluation (the WENO5 smoothness indicators, the PPM parabola and the MUSCL
+// slope of a cell serve its low and its high face), where an evaluation per
+// face (face_at) makes each of them twice.  x and y: a thread walks along the
+// direction, so the high-face values of one cell are the left states of the
+// next face.  z: the 32 lanes of a warp hold 32 neighbouring cells and hand
+// their high-face values to the next lane (31 faces per warp).  Both pass
+// them through shared memory, [variable][thread], which keeps the 18 registers
+// free while the Riemann problem is solved.
+//
+// Divisions: the arithmetic type is fd (one reciprocal per shared
+// denominator); WENO5 takes one per face value, its weights written over a
+// common denominator.  A face with a result that is not finite, or whose WENO5
+// denominators leave [0, 1e300], is evaluated again by the general face_at in
+// float64 with IEEE divisions, so overflows end as they do there.
+//
+// The reference's carried x faces (core/rmhd_core.py:1445,1468) differ from the
+// ordinary ones in the wave speeds alone, so both fluxes are formed from one
+// pair of states instead of by two passes.
+//
+// Bound: the float64 pipe (about 850 float64 operations per RMHD WENO5 face) at 16
+// warps per SM, 128 registers.  One stage's faces of 134^3 cells, RMHD WENO5 "hlld"
+// with carried x faces: 2204 us as four per-face passes with IEEE divisions, 574 us
+// here; SRHD PPM HLLC 377 us, 247 us.
+#include "face64.cuh"
+
+#include <stdint.h>
+
+using namespace astro;
+
+namespace astro_face64 {
+namespace {
+
+constexpr int T = 128;  // threads per block
+
+// face_at as a call: rare, so it must not cost the caller registers
+template <int PHYS, int RECON, int RIEMANN, bool GIVEN, int DIR>
+__device__ __noinline__ void general_face(const Args& a, int i, int j, int k) {
+    FaceArgs f;
+    f.pr = a.pr;
+    f.nx = a.nx; f.ny = a.ny; f.nz = a.nz;
+    f.b = a.b;
+    f.F = GIVEN ? a.FxC : a.F[DIR];
+    f.aux = GIVEN ? nullptr : a.aux[DIR];
+    f.speeds_out = DIR == 2 ? a.speeds_out : nullptr;
+    f.carried = a.carried;
+    f.ndiss = a.ndiss;
+    f.p = a.p;
+    face_at<PHYS, RECON, RIEMANN, double, double, GIVEN, DIR>(f, i, j, k);
+}
+
+// Both WENO5 face values of the cell with stencil q[0..4]: lo is the reference's
+// right-biased value at its low face, hi the left-biased one at its high face.
+// With the differences d_k of neighbouring cells the second differences are t
+// and half the first-derivative terms of the indicators h, so
+// IS_k = 13/12 t^2 + h^2; the candidate polynomials less q[2] are r.  With
+// D_k = (eps + IS_k)^2 the normalised weights g_k / D_k / sum are
+// g_k prod(D_other) / sum, one division per face value instead of six.
+__device__ __forceinline__ void weno5_cell(const double* q, double& lo, double& hi, bool& wide) {
+    const double d0 = q[1] - q[0], d1 = q[2] - q[1], d2 = q[3] - q[2], d3 = q[4] - q[3];
+    const double t0 = d1 - d0, t1 = d2 - d1, t2 = d3 - d2;
+    const double h0 = fma(0.5, t0, d1), h1 = 0.5 * (d1 + d2), h2 = fma(0.5, t2, -d2);
+    constexpr double c = 13.0 / 12.0, eps = 1e-12;
+    const double e0 = fma(c * t0, t0, fma(h0, h0, eps));
+    const double e1 = fma(c * t1, t1, fma(h1, h1, eps));
+    const double e2 = fma(c * t2, t2, fma(h2, h2, eps));
+    const double D0 = e0 * e0, D1 = e1 * e1, D2 = e2 * e2;
+    const double P12 = D1 * D2, P02 = 6.0 * (D0 * D2), P01 = D0 * D1;
+    // weights 1, 6, 3 (the reference's 0.1, 0.6, 0.3 times ten)
+    const double denh = fma(3.0, P01, P12 + P02), denl = fma(3.0, P12, P01 + P02);
+    const double numh = fma(P12, fma(5.0 / 6.0, d1, -1.0 / 3.0 * d0),
+                            fma(P02, fma(1.0 / 6.0, d1, 1.0 / 3.0 * d2), P01 * fma(2.0, d2, -0.5 * d3)));
+    const double numl = fma(P01, fma(-5.0 / 6.0, d2, 1.0 / 3.0 * d3),
+                            fma(P02, fma(-1.0 / 6.0, d2, -1.0 / 3.0 * d1), P12 * fma(-2.0, d1, 0.5 * d0)));
+    // 1e300 by exponent (the sign is clear; infinities and NaN are above)
+    wide |= __double2hiint(denh) >= 0x7e37e43c || __double2hiint(denl) >= 0x7e37e43c;
+    hi = fma(numh, rcp_(fd(denh)).v, q[2]);
+    lo = fma(numl, rcp_(fd(denl)).v, q[2]);
+}
+
+template <int RECON>
+__device__ __forceinline__ void recon_cell(const double* q, int lim, double& lo, double& hi, bool& wide) {
+    if constexpr (RECON == ASTRO_RECON_MUSCL) {
+        const double s = limiter(lim, fd(q[2] - q[1]), fd(q[3] - q[2])).v;
+        lo = q[2] - 0.5 * s;
+        hi = q[2] + 0.5 * s;
+    } else if constexpr (RECON == ASTRO_RECON_PPM) {
+        ppm(q[0], q[1], q[2], q[3], q[4], lo, hi);
+    } else {
+        weno5_cell(q, lo, hi, wide);
+    }
+}
+
+// The cell (i, j, k): its face values, and the flux through its low face in
+// direction DIR (when `face`) from the left states in sh[v * T + thread], which
+// its own high-face values replace.  wide_left: whether the left states'
+// reconstruction left its range; the cell's own on return.
+template <int PHYS, int RECON, int RIEMANN, int DIR>
+__device__ __forceinline__ void cell_and_face(const Args& a, double* sh, int i, int j, int k, bool face,
+                                              bool& wide_left) {
+    constexpr int NM = PHYS == ASTRO_SRHD ? 5 : 9;
+    const int t = threadIdx.x;
+    const size_t nc = (size_t)a.nx * a.ny * a.nz;
+    const size_t cell = ((size_t)i * a.ny + j) * a.nz + k;
+    const long stride = DIR == 0 ? (long)a.ny * a.nz : (DIR == 1 ? (long)a.nz : 1L);
+    constexpr int w = RECON == ASTRO_RECON_MUSCL ? 1 : 2;
+    bool wide = false;
+    fd qL[NM], qR[NM];
+#pragma unroll
+    for (int v = 0; v < NM; ++v) {
+        double q[5], lo, hi;
+        const double* base = a.pr + (size_t)v * nc + cell;
+#pragma unroll
+        for (int o = -w; o <= w; ++o) q[o + 2] = __ldg(base + o * stride);
+        recon_cell<RECON>(q, a.p.limiter, lo, hi, wide);
+        qR[v] = fd(lo);
+        if constexpr (DIR != 2) qL[v] = fd(sh[v * T + t]);
+        sh[v * T + t] = hi;
+    }
+    if constexpr (DIR == 2) {
+        // the lane below holds the cell below
+        wide_left = __any_sync(0xffffffffu, wide);
+        __syncwarp();
+#pragma unroll
+        for (int v = 0; v < NM; ++v) qL[v] = fd(sh[v * T + t - (t & 31 ? 1 : 0)]);
+    }
+    const bool wide_here = wide;
+    wide |= wide_left;
+    wide_left = wide_here;
+    if (!face) return;
+    const Phys<fd> P = Phys<fd>::from(a.p);
+    fd F[NM], sL, sR;
+    double* Fo = a.F[DIR];
+    bool ok = !wide;
+    if constexpr (PHYS == ASTRO_SRHD) {
+        if (RECON == ASTRO_RECON_MUSCL && a.p.passive_offset > 5) {
+            // add_pi_lr (srhd_core.py:394-398), as in face_at
+            qL[4] += fd(__ldg(a.pr + 5 * nc + cell - stride));
+            qR[4] += fd(__ldg(a.pr + 5 * nc + cell));
+        }
+        if (a.ndiss > 0) {
+            fd isL[10], isR[10];
+#pragma unroll
+            for (int m = 0; m < 10; ++m) {
+                isL[m] = fd(__ldg(a.pr + (size_t)(5 + m) * nc + cell - stride));
+                isR[m] = fd(__ldg(a.pr + (size_t)(5 + m) * nc + cell));
+            }
+            s_face<RIEMANN>(P, DIR, qL, qR, F, sL, sR, a.ndiss, isL, isR);
+        } else {
+            s_face<RIEMANN>(P, DIR, qL, qR, F, sL, sR);
+        }
+    } else {
+        constexpr bool OVR = RECON == ASTRO_RECON_MUSCL;
+        fd UL[9], UR[9], FL[9], FR[9];
+        r_face_states(P, DIR, qL, qR, UL, UR, FL, FR, sL, sR);
+        r_riemann<RIEMANN, OVR>(P, DIR, qL, qR, UL, UR, FL, FR, sL, sR, F);
+        if (DIR == 0 && !OVR && a.FxC && i < a.b.hi[0]) {
+            // the x-low face of an updated cell with the z-face speeds left
+            // over from the previous cell of the reference's i-j-k loop
+            double cL = -1.0, cR = 1.0;
+            int pi = i, pj = j, pk = k - 1;
+            if (k == a.b.lo) {
+                pk = a.b.hi[2] - 1;
+                if (j > a.b.lo) pj = j - 1;
+                else { pj = a.b.hi[1] - 1; pi = i - 1; }
+            }
+            if (pi >= a.b.lo) {
+                const size_t pc = ((size_t)pi * a.ny + pj) * a.nz + pk;
+                cL = a.carried[pc];
+                cR = a.carried[nc + pc];
+            }
+            fd G[9];
+            r_riemann<RIEMANN, OVR>(P, 0, qL, qR, UL, UR, FL, FR, fd(cL), fd(cR), G);
+            bool okc = !wide;
+#pragma unroll
+            for (int v = 0; v < 9; ++v) {
+                okc &= isfinite(G[v].v);
+                a.FxC[(size_t)v * nc + cell] = G[v].v;
+            }
+            if (!okc) general_face<PHYS, RECON, RIEMANN, DIR == 0 && !OVR, 0>(a, i, j, k);
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < NM; ++v) {
+        ok &= isfinite(F[v].v);
+        Fo[(size_t)v * nc + cell] = F[v].v;
+    }
+    ok &= isfinite(sL.v) && isfinite(sR.v);
+    if (a.aux[DIR]) {
+        double* A = a.aux[DIR];
+        A[cell] = sL.v;
+        A[nc + cell] = sR.v;
+        A[2 * nc + cell] = qL[1 + DIR].v;
+        A[3 * nc + cell] = qR[1 + DIR].v;
+    }
+    if (DIR == 2 && a.speeds_out) {
+        a.speeds_out[cell] = sL.v;
+        a.speeds_out[nc + cell] = sR.v;
+    }
+    if (!ok) general_face<PHYS, RECON, RIEMANN, false, DIR>(a, i, j, k);
+}
+
+// threads of direction DIR (0, 1): the plane across it, times segments of
+// a.seg[DIR] faces along it
+template <int PHYS, int RECON, int RIEMANN, int DIR>
+__device__ __forceinline__ void walk(const Args& a, double* sh, unsigned block) {
+    const int lo = a.b.lo;
+    const unsigned e2 = (unsigned)(a.b.hi[2] - lo);
+    const unsigned eo = (unsigned)(a.b.hi[DIR == 0 ? 1 : 0] - lo);
+    const unsigned plane = e2 * eo;
+    const unsigned per = (plane + T - 1) / T;  // blocks per segment
+    const unsigned sg = block / per, tp = (block - sg * per) * T + threadIdx.x;
+    if (tp >= plane) return;
+    const int k = lo + (int)(tp % e2), o = lo + (int)(tp / e2);
+    const int f0 = lo + (int)sg * a.seg[DIR];
+    int f1 = f0 + a.seg[DIR];
+    if (f1 > a.b.hi[DIR] + 1) f1 = a.b.hi[DIR] + 1;
+    // the first turn only makes the left states of face f0
+    bool wide = false;
+    for (int f = f0 - 1; f < f1; ++f)
+        cell_and_face<PHYS, RECON, RIEMANN, DIR>(a, sh, DIR == 0 ? f : o, DIR == 0 ? o : f, k, f >= f0,
+                                                 wide);
+}
+
+template <int PHYS, int RECON, int RIEMANN>
+__global__ void __launch_bounds__(T, RIEMANN == ASTRO_RIEMANN_HLLD_FULL ? 2 : 4)
+    k_face64(const __grid_constant__ Args a) {
+    constexpr int NM = PHYS == ASTRO_SRHD ? 5 : 9;
+    __shared__ double sh[NM * T];
+    if (blockIdx.x < (unsigned)a.blocks_z) {
+        // one warp per 31 z faces of a row: lane 0 only makes left states
+        const int lo = a.b.lo, faces = a.b.hi[2] - lo + 1;
+        const unsigned per = (unsigned)(faces + 30) / 31;
+        const unsigned wp = blockIdx.x * (T / 32) + threadIdx.x / 32;
+        const unsigned r = wp / per, ey = (unsigned)(a.b.hi[1] - lo);
+        const int i = lo + (int)(r / ey), j = lo + (int)(r % ey);
+        if (i >= a.b.hi[0]) return;
+        const int k = lo + (int)(wp % per) * 31 + (int)(threadIdx.x & 31) - 1;
+        // lanes past the last face repeat its cell, without a face
+        bool wide = false;
+        cell_and_face<PHYS, RECON, RIEMANN, 2>(a, sh, i, j, k < a.b.hi[2] ? k : a.b.hi[2],
+                                               (threadIdx.x & 31) > 0 && k <= a.b.hi[2], wide);
+    } else if (blockIdx.x < (unsigned)(a.blocks_z + a.blocks_y)) {
+        walk<PHYS, RECON, RIEMANN, 1>(a, sh, blockIdx.x - a.blocks_z);
+    } else {
+        walk<PHYS, RECON, RIEMANN, 0>(a, sh, blockIdx.x - a.blocks_z - a.blocks_y);
+    }
+}
+
+template <int PH, int RE>
+void launch_riemann(const Args& a, unsigned blocks, cudaStream_t s) {
+    if (a.p.riemann == 0) k_face64<PH, RE, 0><<<blocks, T, 0, s>>>(a);
+    else if (a.p.riemann == 1) k_face64<PH, RE, 1><<<blocks, T, 0, s>>>(a);
+    else if constexpr (PH == ASTRO_RMHD) k_face64<PH, RE, 2><<<blocks, T, 0, s>>>(a);
+}
+
+}  // namespace
+
+cudaError_t launch(Args a, int sms, cudaStream_t s) {
+    const long e[3] = {a.b.hi[0] - a.b.lo, a.b.hi[1] - a.b.lo, a.b.hi[2] - a.b.lo};
+    if (e[0] <= 0 || e[1] <= 0 || e[2] <= 0) return cudaSuccess;
+    long blocks[3] = {0, 0, 0};
+    if (a.F[2]) blocks[2] = (e[0] * e[1] * ((e[2] + 1 + 30) / 31) + T / 32 - 1) / (T / 32);
+    for (int d = 0; d < 2; ++d) {
+        if (!a.F[d]) continue;
+        // A longer walk repeats fewer reconstructions at its start (1 per
+        // segment); a shorter one gives more threads.  Four times the resident
+        // threads (4 blocks per SM) keep the last wave small; up to 16 faces per
+        // thread, where the repeated share is 6 %.
+        const long plane = e[1 - d] * e[2], faces = e[d] + 1;
+        long seg = plane * faces / ((long)sms * 4 * T * 4);
+        if (seg < 1) seg = 1;
+        if (seg > 16) seg = 16;
+        a.seg[d] = (int)seg;
+        blocks[d] = ((plane + T - 1) / T) * ((faces + seg - 1) / seg);
+    }
+    a.blocks_z = (int)blocks[2];
+    a.blocks_y = (int)blocks[1];
+    const long total = blocks[0] + blocks[1] + blocks[2];
+    if (total == 0) return cudaSuccess;
+    if (total > 0x7fffffffL) return cudaErrorInvalidValue;
+    const unsigned n = (unsigned)total;
+    if (a.p.physics == ASTRO_SRHD) {
+        if (a.p.recon == 0) launch_riemann<ASTRO_SRHD, 0>(a, n, s);
+        else if (a.p.recon == 1) launch_riemann<ASTRO_SRHD, 1>(a, n, s);
+        else launch_riemann<ASTRO_SRHD, 2>(a, n, s);
+    } else {
+        if (a.p.recon == 0) launch_riemann<ASTRO_RMHD, 0>(a, n, s);
+        else if (a.p.recon == 1) launch_riemann<ASTRO_RMHD, 1>(a, n, s);
+        else launch_riemann<ASTRO_RMHD, 2>(a, n, s);
+    }
+    return cudaGetLastError();
+}
+
+}  // namespace astro_face64

@@ -1,0 +1,26 @@
+// face64.cuh -- the float64 face passes (interface between face64.cu and
+// kernels.cu; not part of the C ABI).
+#pragma once
+#include "face.cuh"
+
+namespace astro_face64 {
+
+// the faces of up to three directions of one block in one launch
+struct Args {
+    const double* pr;
+    int nx, ny, nz;
+    astro::Bounds b;     // updated cells; the faces on both sides of each
+    double* F[3];        // fluxes per direction, [nm][nc]; null: not this launch
+    double* aux[3];      // sL, sR, vL, vR per direction, or null
+    double* speeds_out;  // z faces: sL, sR for the carried x faces, or null
+    double* FxC;         // x faces: also the fluxes with the carried speeds, or null
+    const double* carried;  // those speeds (an earlier launch's speeds_out)
+    int ndiss;
+    AstroParams p;
+    // set by launch(): thread blocks of z, y (x follow) and faces per thread
+    int blocks_z, blocks_y, seg[2];
+};
+
+cudaError_t launch(Args a, int sms, cudaStream_t s);
+
+}  // namespace astro_face64

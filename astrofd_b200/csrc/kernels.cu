@@ -1,12 +1,13 @@
 // kernels.cu -- sm_100a kernels and the C ABI of libastrofd_b200.so.
 //
 // Per SSPRK stage the right-hand side is built face by face:
-//   k_face    one thread per cell face in one direction: reconstruct the
-//             left/right primitive states from the 4- or 6-point stencil,
-//             floor, p2c, physical flux, wave speeds, Riemann flux.  Every face
-//             is evaluated once (the reference evaluates each face twice, once
-//             from each neighbour).  The result lands in a per-direction face
-//             buffer F[v][cell], indexed by the cell on the high side.
+//   faces     reconstruct the left/right primitive states from the 4- or 6-point
+//             stencil, floor, p2c, physical flux, wave speeds, Riemann flux:
+//             float32 one thread per face (face32.cu), float64 cell by cell
+//             along the direction (face64.cu).  Every face is evaluated once
+//             (the reference evaluates each face twice, once from each
+//             neighbour).  The result lands in a per-direction face buffer
+//             F[v][cell], indexed by the cell on the high side.
 //   k_update  one thread per cell (ghosts included): flux divergence, GLM
 //             damping, resistive Laplacian, passive-scalar fluxes, the SSPRK
 //             combination in float64 and con2prim, writing U_k and the next
@@ -14,10 +15,11 @@
 //             rhs = 0, i.e. the reference's p2c -> c2p round trip.
 // The reference's RMHD PPM/WENO x faces use the wave speeds left over from the
 // previous cell's z face (core/rmhd_core.py:1285,1314,1445,1468).  In
-// ASTRO_FLUX_REFERENCE mode those faces are evaluated a second time with the
-// carried speeds (k_face<GIVEN=true>), read from the z-face speed buffer; in
-// ASTRO_FLUX_CONSERVATIVE mode every face uses its own speeds, so each face
-// flux enters both neighbours and the scheme conserves D, S, tau exactly.
+// ASTRO_FLUX_REFERENCE mode those faces get a second flux with the carried
+// speeds, read from the z-face speed buffer (float32: a second pass, k_face<GIVEN>;
+// float64: from the same states in the same pass); in ASTRO_FLUX_CONSERVATIVE mode
+// every face uses its own speeds, so each face flux enters both neighbours and
+// the scheme conserves D, S, tau exactly.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -26,6 +28,9 @@
 #include <mutex>
 #include <vector>
 
+#include "face.cuh"
+#include "face32.cuh"
+#include "face64.cuh"
 #include "mlp.cuh"
 #include "physics.cuh"
 #include "stage.cuh"
@@ -100,10 +105,6 @@ inline void mark(int kind, cudaStream_t s) {
 
 constexpr int kMaxPassive = 8;
 constexpr int kMaxNV = 64;
-
-struct Bounds {
-    int lo, hi[3];  // cells updated: [lo, hi[d]) per dimension
-};
 
 // loop bounds of the reference right-hand sides (ghost-inclusive indices)
 __host__ Bounds bounds_of(const AstroParams& p, const AstroGrid& g) {
@@ -214,195 +215,6 @@ int validate(const AstroParams* p, const AstroGrid* g) {
 }
 
 // ------------------------------------------------------------ face pass ---
-struct FaceArgs {
-    const double* pr;
-    const float* prf;    // float32 copy of the nm primitives (float32 passes)
-    int nx, ny, nz;
-    int dir;
-    int org[3], ext[3];  // first cell and extents of the face block
-    Bounds b;
-    void* F;             // R[nm][nc]
-    void* aux;           // R[4][nc]: sL, sR, vL, vR (or null)
-    void* speeds_out;    // R[2][nc]: sL, sR (z faces, carried mode) or null
-    const void* carried; // R[2][nc]: z-face speeds read by the carried x faces
-    int ndiss;           // SRHD Israel-Stewart blocks: dissipation fluxes per face
-    AstroParams p;
-    // float32 passes: faces whose float32 result is not finite are listed here
-    // and recomputed in float64 by k_face_fix
-    unsigned* fix_count;
-    unsigned* fix_list;
-    unsigned fix_cap;
-};
-
-// One face: reconstruct, floor, p2c, flux, speeds, Riemann in arithmetic R,
-// stored as RS.  Returns false when the stored flux or speeds are not finite.
-template <int PHYS, int RECON, int RIEMANN, typename R, typename RS, bool GIVEN, int DIR>
-__device__ __forceinline__ bool face_at(const FaceArgs& a, int i, int j, int k) {
-    constexpr int NM = PHYS == ASTRO_SRHD ? 5 : 9;
-    const size_t nc = (size_t)a.nx * a.ny * a.nz;
-    const size_t cell = ((size_t)i * a.ny + j) * a.nz + k;
-    const long stride = DIR == 0 ? (long)a.ny * a.nz : (DIR == 1 ? (long)a.nz : 1L);
-    const Phys<R> P = Phys<R>::from(a.p);
-
-    R qL[NM], qR[NM];
-    constexpr int o0 = RECON == ASTRO_RECON_MUSCL ? -2 : -3;
-    constexpr int o1 = RECON == ASTRO_RECON_MUSCL ? 1 : 2;
-#pragma unroll
-    for (int v = 0; v < NM; ++v) {
-        R st[6];
-        if constexpr (sizeof(R) == 4) {
-            // the float32 copy: one conversion per cell and stage instead of
-            // one per stencil use
-            const float* base = a.prf + (size_t)v * nc + cell;
-#pragma unroll
-            for (int o = o0; o <= o1; ++o) st[o + 3] = __ldg(base + o * stride);
-        } else {
-            const double* base = a.pr + (size_t)v * nc + cell;
-#pragma unroll
-            for (int o = o0; o <= o1; ++o) st[o + 3] = (R)__ldg(base + o * stride);
-        }
-        recon_face<RECON>(st, a.p.limiter, qL[v], qR[v]);
-    }
-    R F[NM];
-    R sL = R(-1), sR = R(1);
-    if (GIVEN) {
-        // previous cell of the reference's i-j-k loop, whose z-low face speeds
-        // are still in (sL, sR) when this cell's x-low face is evaluated
-        int pi = i, pj = j, pk = k;
-        bool first = false;
-        if (k > a.b.lo) pk = k - 1;
-        else if (j > a.b.lo) { pj = j - 1; pk = a.b.hi[2] - 1; }
-        else if (i > a.b.lo) { pi = i - 1; pj = a.b.hi[1] - 1; pk = a.b.hi[2] - 1; }
-        else first = true;
-        if (!first) {
-            const RS* S = (const RS*)a.carried;
-            const size_t pc = ((size_t)pi * a.ny + pj) * a.nz + pk;
-            sL = (R)S[pc];
-            sR = (R)S[nc + pc];
-        }
-    }
-    if (PHYS == ASTRO_SRHD) {
-        if (RECON == ASTRO_RECON_MUSCL && a.p.passive_offset > 5) {
-            // add_pi_lr (srhd_core.py:394-398): the cells' bulk pressure on
-            // the reconstructed face pressures, before the floor
-            qL[4] += (R)__ldg(a.pr + 5 * nc + cell - stride);
-            qR[4] += (R)__ldg(a.pr + 5 * nc + cell);
-        }
-        if (a.ndiss > 0) {
-            R isL[10], isR[10];
-#pragma unroll
-            for (int m = 0; m < 10; ++m) {
-                isL[m] = (R)__ldg(a.pr + (size_t)(5 + m) * nc + cell - stride);
-                isR[m] = (R)__ldg(a.pr + (size_t)(5 + m) * nc + cell);
-            }
-            s_face<RIEMANN>(P, DIR, qL, qR, F, sL, sR, a.ndiss, isL, isR);
-        } else {
-            s_face<RIEMANN>(P, DIR, qL, qR, F, sL, sR);
-        }
-    } else {
-        r_face<RIEMANN, RECON == ASTRO_RECON_MUSCL, GIVEN>(P, DIR, qL, qR, F, sL, sR);
-    }
-    RS* Fo = (RS*)a.F;
-    bool finite = true;
-#pragma unroll
-    for (int v = 0; v < NM; ++v) {
-        const RS f = (RS)F[v];
-        finite &= isfinite(f);
-        Fo[(size_t)v * nc + cell] = f;
-    }
-    finite &= isfinite((RS)sL) && isfinite((RS)sR);
-    if (a.aux) {
-        RS* A = (RS*)a.aux;
-        A[cell] = (RS)sL;
-        A[nc + cell] = (RS)sR;
-        A[2 * nc + cell] = (RS)qL[1 + DIR];
-        A[3 * nc + cell] = (RS)qR[1 + DIR];
-    }
-    if (a.speeds_out) {
-        RS* S = (RS*)a.speeds_out;
-        S[cell] = (RS)sL;
-        S[nc + cell] = (RS)sR;
-    }
-    return finite;
-}
-
-template <int PHYS, int RECON, int RIEMANN, typename R, bool GIVEN, int DIR>
-__global__ void __launch_bounds__(128) k_face(FaceArgs a) {
-    // grid: x over the (j, k) plane of the face block, y over its x layers;
-    // one 32-bit split of the in-plane index per thread
-    const unsigned e2 = (unsigned)a.ext[2];
-    const unsigned plane = (unsigned)a.ext[1] * e2;
-    const unsigned tp = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tp >= plane) return;
-    const int c = (int)(tp % e2), bb = (int)(tp / e2);
-    for (int aa = blockIdx.y; aa < a.ext[0]; aa += gridDim.y) {
-        const int i = a.org[0] + aa, j = a.org[1] + bb, k = a.org[2] + c;
-        const bool ok = face_at<PHYS, RECON, RIEMANN, R, R, GIVEN, DIR>(a, i, j, k);
-        if (sizeof(R) == 4 && !ok && a.fix_list) {
-            const unsigned slot = atomicAdd(a.fix_count, 1u);
-            if (slot < a.fix_cap) a.fix_list[slot] = (unsigned)aa * plane + tp;
-        }
-    }
-}
-
-// whether everything face_at stored for this face (fluxes, and the speeds
-// and face velocities where the pass keeps them) is finite
-template <int NM>
-__device__ __forceinline__ bool face_stored_finite(const FaceArgs& a, size_t nc, size_t cell) {
-    bool ok = true;
-    const float* F = (const float*)a.F;
-#pragma unroll
-    for (int v = 0; v < NM; ++v) ok &= isfinite(F[(size_t)v * nc + cell]);
-    if (a.aux) {
-        const float* A = (const float*)a.aux;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) ok &= isfinite(A[(size_t)m * nc + cell]);
-    }
-    if (a.speeds_out) {
-        const float* S = (const float*)a.speeds_out;
-        ok &= isfinite(S[cell]) && isfinite(S[nc + cell]);
-    }
-    return ok;
-}
-
-// float64 recomputation of the faces a float32 pass listed as non-finite
-// (float32 overflows where float64 does not, e.g. squared WENO smoothness
-// indicators of a state whose fields have grown past ~1e9).  If more faces
-// failed than the list holds (the counter keeps counting past its capacity),
-// the list is incomplete: every face of the pass is then checked and the
-// non-finite ones are recomputed, so no float32 failure is left in place.
-template <int PHYS, int RECON, int RIEMANN, bool GIVEN, int DIR>
-__global__ void __launch_bounds__(128) k_face_fix(FaceArgs a) {
-    constexpr int NM = PHYS == ASTRO_SRHD ? 5 : 9;
-    const unsigned cnt = *a.fix_count;
-    if (cnt <= a.fix_cap) {
-        for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < cnt;
-             q += gridDim.x * blockDim.x) {
-            const long t = a.fix_list[q];
-            const int c = (int)(t % a.ext[2]);
-            const long r = t / a.ext[2];
-            const int bb = (int)(r % a.ext[1]);
-            const int aa = (int)(r / a.ext[1]);
-            face_at<PHYS, RECON, RIEMANN, double, float, GIVEN, DIR>(a, a.org[0] + aa,
-                                                                    a.org[1] + bb, a.org[2] + c);
-        }
-        return;
-    }
-    const size_t nc = (size_t)a.nx * a.ny * a.nz;
-    const size_t plane = (size_t)a.ext[1] * a.ext[2];
-    const size_t total = (size_t)a.ext[0] * plane;
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < total;
-         q += (size_t)gridDim.x * blockDim.x) {
-        const int aa = (int)(q / plane);
-        const size_t tp = q % plane;
-        const int bb = (int)(tp / a.ext[2]), c = (int)(tp % a.ext[2]);
-        const int i = a.org[0] + aa, j = a.org[1] + bb, k = a.org[2] + c;
-        const size_t cell = ((size_t)i * a.ny + j) * a.nz + k;
-        if (!face_stored_finite<NM>(a, nc, cell))
-            face_at<PHYS, RECON, RIEMANN, double, float, GIVEN, DIR>(a, i, j, k);
-    }
-}
-
 // ---------------------------------------------------------- update pass ---
 struct UpdArgs {
     const double* pr0;   // step input primitives (U0 = p2c(pr0), passives t0)
@@ -967,69 +779,6 @@ __global__ void k_prim_f32_rows(const double* __restrict__ pr, float* __restrict
 }
 
 // ------------------------------------------------------------- dispatch ---
-// direction is a template parameter so the per-direction component indices
-// fold to constants and the face state stays in registers
-template <int PH, int RE, int RI, typename R>
-cudaError_t launch_face_dir(const FaceArgs& a, bool given, dim3 grd, dim3 blk, cudaStream_t s) {
-    constexpr bool F32 = sizeof(R) == 4;
-    const dim3 fgrd(148 * 4);
-    // the fix-up counter starts every float32 pass at zero (the workspace, or
-    // the shared static scratch, holds the previous pass's count)
-    if (F32) {
-        const cudaError_t e = cudaMemsetAsync(a.fix_count, 0, sizeof(unsigned), s);
-        if (e != cudaSuccess) return e;
-    }
-    if constexpr (PH == ASTRO_RMHD && RE != ASTRO_RECON_MUSCL) {
-        if (given) {
-            k_face<PH, RE, RI, R, true, 0><<<grd, blk, 0, s>>>(a);
-            if (F32) k_face_fix<PH, RE, RI, true, 0><<<fgrd, blk, 0, s>>>(a);
-            return cudaSuccess;
-        }
-    }
-    if (a.dir == 0) {
-        k_face<PH, RE, RI, R, false, 0><<<grd, blk, 0, s>>>(a);
-        if (F32) k_face_fix<PH, RE, RI, false, 0><<<fgrd, blk, 0, s>>>(a);
-    } else if (a.dir == 1) {
-        k_face<PH, RE, RI, R, false, 1><<<grd, blk, 0, s>>>(a);
-        if (F32) k_face_fix<PH, RE, RI, false, 1><<<fgrd, blk, 0, s>>>(a);
-    } else {
-        k_face<PH, RE, RI, R, false, 2><<<grd, blk, 0, s>>>(a);
-        if (F32) k_face_fix<PH, RE, RI, false, 2><<<fgrd, blk, 0, s>>>(a);
-    }
-    return cudaSuccess;
-}
-
-template <typename R>
-cudaError_t launch_face_t(const FaceArgs& a, bool given, cudaStream_t s) {
-    // an empty cell range in any direction: no faces (checked per extent,
-    // since two negative extents would give a positive product)
-    if (a.ext[0] <= 0 || a.ext[1] <= 0 || a.ext[2] <= 0) return cudaSuccess;
-    const unsigned plane = (unsigned)a.ext[1] * (unsigned)a.ext[2];
-    const dim3 blk(128), grd((plane + 127) / 128, (unsigned)(a.ext[0] < 65535 ? a.ext[0] : 65535));
-    const AstroParams& p = a.p;
-    cudaError_t me = cudaSuccess;
-#define FACE(PH, RE, RI) me = launch_face_dir<PH, RE, RI, R>(a, given, grd, blk, s)
-#define RECONS(PH, RI)                                                          \
-    do {                                                                        \
-        if (p.recon == 0) FACE(PH, 0, RI);                                      \
-        else if (p.recon == 1) FACE(PH, 1, RI);                                 \
-        else FACE(PH, 2, RI);                                                   \
-    } while (0)
-    if (p.physics == ASTRO_SRHD) {
-        if (p.riemann == 1) RECONS(ASTRO_SRHD, 1);
-        else RECONS(ASTRO_SRHD, 0);
-    } else {
-        if (p.riemann == 2) RECONS(ASTRO_RMHD, 2);
-        else if (p.riemann == 1) RECONS(ASTRO_RMHD, 1);
-        else RECONS(ASTRO_RMHD, 0);
-    }
-#undef RECONS
-#undef FACE
-    if (me != cudaSuccess) return me;
-    mark(0, s);
-    return cudaGetLastError();
-}
-
 template <int PH, typename RF, bool DEF, bool PAS>
 void launch_update_t(const UpdArgs& a, dim3 grd, dim3 blk, cudaStream_t s) {
     k_update<PH, RF, DEF, PAS><<<grd, blk, 0, s>>>(a);
@@ -1085,6 +834,32 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
         k_prim_f32<<<sm_count_cached() * 8, 256, 0, s>>>(pr, prf, n);
         mark(2, s);
     }
+    if (!mixed) {
+        // one launch for all directions; the carried x faces need the z
+        // faces' speeds, so there x follows in a second one
+        astro_face64::Args a;
+        memset(&a, 0, sizeof(a));
+        a.pr = pr; a.nx = g.nx; a.ny = g.ny; a.nz = g.nz; a.b = b; a.p = p;
+        a.ndiss = dissipation_fluxes(p, g);
+        for (int d = 0; d < 3; ++d) {
+            if (d > 0 || !carried) a.F[d] = (double*)(work + L.F[d]);
+            a.aux[d] = passive_fluxes(p) ? (double*)(work + L.aux[d]) : nullptr;
+        }
+        if (carried) a.speeds_out = (double*)(work + L.Sz);
+        cudaError_t e = astro_face64::launch(a, sm_count_cached(), s);
+        if (e != cudaSuccess) return e;
+        mark(0, s);
+        if (!carried) return cudaSuccess;
+        a.F[0] = (double*)(work + L.F[0]);
+        a.F[1] = a.F[2] = nullptr;
+        a.speeds_out = nullptr;
+        a.FxC = (double*)(work + L.FxC);
+        a.carried = (const double*)(work + L.Sz);
+        e = astro_face64::launch(a, sm_count_cached(), s);
+        if (e != cudaSuccess) return e;
+        mark(0, s);
+        return cudaSuccess;
+    }
     for (int oi = 0; oi < 3; ++oi) {
         const int d = order[oi];
         FaceArgs a;
@@ -1097,14 +872,13 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
         }
         a.F = work + L.F[d];
         a.aux = passive_fluxes(p) ? (void*)(work + L.aux[d]) : nullptr;
-        if (mixed) {
-            a.fix_count = (unsigned*)(work + L.fix);
-            a.fix_list = (unsigned*)(work + L.fix + 256);
-            a.fix_cap = (unsigned)fix_capacity(g);
-        }
+        a.fix_count = (unsigned*)(work + L.fix);
+        a.fix_list = (unsigned*)(work + L.fix + 256);
+        a.fix_cap = (unsigned)fix_capacity(g);
         a.speeds_out = (carried && d == 2) ? (void*)(work + L.Sz) : nullptr;
-        cudaError_t e = mixed ? launch_face_t<float>(a, false, s) : launch_face_t<double>(a, false, s);
+        cudaError_t e = astro_face32::launch(a, false, s);
         if (e != cudaSuccess) return e;
+        mark(0, s);
         if (carried && d == 0) {
             FaceArgs c = a;
             c.ext[0] = b.hi[0] - b.lo;  // x-low faces of the updated cells
@@ -1112,8 +886,9 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
             c.aux = nullptr;
             c.speeds_out = nullptr;
             c.carried = work + L.Sz;
-            e = mixed ? launch_face_t<float>(c, true, s) : launch_face_t<double>(c, true, s);
+            e = astro_face32::launch(c, true, s);
             if (e != cudaSuccess) return e;
+            mark(0, s);
         }
     }
     return cudaSuccess;

@@ -24,6 +24,33 @@
 
 namespace astro {
 
+// Float64 whose divisions and square roots are formed from reciprocals (below),
+// for the faces of the float64 path; the same 8 bytes and the same additions
+// and multiplications as double.
+struct fd {
+    double v;
+    fd() = default;
+    AHD constexpr fd(double x) : v(x) {}
+    AHD explicit constexpr operator double() const { return v; }
+};
+AHD fd operator+(fd a, fd b) { return fd(a.v + b.v); }
+AHD fd operator-(fd a, fd b) { return fd(a.v - b.v); }
+AHD fd operator*(fd a, fd b) { return fd(a.v * b.v); }
+AHD fd operator/(fd a, fd b) { return fd(a.v / b.v); }
+AHD fd operator-(fd a) { return fd(-a.v); }
+AHD fd& operator+=(fd& a, fd b) { a.v += b.v; return a; }
+AHD fd& operator*=(fd& a, fd b) { a.v *= b.v; return a; }
+AHD bool operator<(fd a, fd b) { return a.v < b.v; }
+AHD bool operator>(fd a, fd b) { return a.v > b.v; }
+AHD bool operator<=(fd a, fd b) { return a.v <= b.v; }
+AHD bool operator>=(fd a, fd b) { return a.v >= b.v; }
+AHD bool operator==(fd a, fd b) { return a.v == b.v; }
+
+// arithmetic types that take reciprocals of shared denominators; double keeps
+// the reference's divisions
+template <typename R> constexpr bool kRecip = sizeof(R) == 4;
+template <> constexpr bool kRecip<fd> = true;
+
 template <typename R> struct C {
     static constexpr R small = R(1e-12);
 };
@@ -31,6 +58,7 @@ template <typename R> struct C {
 template <typename R> AHD R rmax(R a, R b) { return a > b ? a : b; }
 template <typename R> AHD R rmin(R a, R b) { return a < b ? a : b; }
 template <typename R> AHD R rsqrt_(R x) { return sqrt(x); }
+AHD fd rsqrt_(fd x);
 template <typename R> AHD R rabs(R x) { return x < R(0) ? -x : x; }
 
 // The float32 face path takes one approximate reciprocal per shared
@@ -78,9 +106,42 @@ AHD double rcp_nr(double x) {
 #endif
 }
 
-// a / b: float32 as a * rcp(b), float64 as the IEEE quotient
+// The fd reciprocal and reciprocal square root: the hardware approximations
+// rcp.approx.ftz.f64 and rsqrt.approx.ftz.f64 (relative error e0 ~ 2^-20) with one
+// third-order step of the series of 1/(1 - e) and 1/sqrt(1 - e),
+//   r (1 + e + e^2),            e = 1 - x r,     remainder e^3,
+//   r (1 + e/2 + 3 e^2 / 8),    e = 1 - x r^2,   remainder 5 e^3 / 16,
+// below 2^-58, so that rounding alone remains (within 2 ulp).  One operation
+// of the multi-function unit and three or five of the float64 pipe, without the
+// range tests and the slow branch of an IEEE division.  For normal arguments:
+// zero, infinity and subnormals give a value that is not finite, which sends
+// the face to the general evaluation.
+template <> AHD fd rcp_(fd x) {
+#ifdef __CUDA_ARCH__
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x.v));
+    const double e = fma(-x.v, r, 1.0);
+    return fd(fma(r, fma(e, e, e), r));
+#else
+    return fd(1.0 / x.v);
+#endif
+}
+template <> AHD fd rsq_(fd x) {
+#ifdef __CUDA_ARCH__
+    double r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x.v));
+    const double e = fma(-(x.v * r), r, 1.0);
+    return fd(fma(r * e, fma(0.375, e, 0.5), r));
+#else
+    return fd(1.0 / sqrt(x.v));
+#endif
+}
+// sqrt(x), x >= 0: x / sqrt(x) with the argument kept off zero
+AHD fd rsqrt_(fd x) { return x * rsq_(rmax(x, fd(1e-290))); }
+
+// a / b: float32 and fd as a * rcp(b), float64 as the IEEE quotient
 template <typename R> AHD R qdiv(R a, R b) {
-    if constexpr (sizeof(R) == 4) return a * rcp_(b);
+    if constexpr (kRecip<R>) return a * rcp_(b);
     else return a / b;
 }
 
@@ -110,7 +171,7 @@ template <typename R> AHD R limiter(int id, R dqL, R dqR) {
         if (dqL * dqR <= R(0)) return R(0);
         R denom = dqL + dqR;
         if (denom == R(0)) return R(0);
-        return (R(2) * dqL * dqR) / denom;
+        return kRecip<R> && sizeof(R) == 8 ? qdiv(R(2) * dqL * dqR, denom) : (R(2) * dqL * dqR) / denom;
     }
     R mm = minmod(dqL, dqR);
     return minmod(R(0.5) * (dqL + dqR), R(2) * mm);
@@ -233,7 +294,7 @@ AHD void hlle(const R* UL, const R* UR, const R* FL, const R* FR, R sL, R sR, R*
     if (sL >= R(0)) { for (int v = V0; v < N; ++v) out[v] = FL[v]; return; }
     if (sR <= R(0)) { for (int v = V0; v < N; ++v) out[v] = FR[v]; return; }
     R inv = sR - sL + C<R>::small;
-    if constexpr (sizeof(R) == 4) {
+    if constexpr (kRecip<R>) {
         const R ri = rcp_(inv);
 #pragma unroll
         for (int v = V0; v < N; ++v) out[v] = (sR * FL[v] - sL * FR[v] + sL * sR * (UR[v] - UL[v])) * ri;
@@ -248,7 +309,7 @@ template <typename R> AHD void eig_speeds(R vn, R cs, R& lm, R& lp) {
     if (dp == R(0)) dp = C<R>::small;
     if (dm == R(0)) dm = C<R>::small;
     R p, m;
-    if constexpr (sizeof(R) == 4) {
+    if constexpr (kRecip<R>) {
         const R r = rcp_(dp * dm);
         p = (vn + cs) * dm * r;
         m = (vn - cs) * dp * r;
@@ -269,7 +330,9 @@ template <typename R> AHD void s_p2c(const Phys<R>& P, const R* q, R* U) {
     R rho = q[0], vx = q[1], vy = q[2], vz = q[3], p = q[4];
     R v2 = vx * vx + vy * vy + vz * vz;
     if (v2 >= R(1)) v2 = R(1) - R(1e-14);
-    R W = sizeof(R) == 4 ? rsq_(R(1) - v2) : R(1) / rsqrt_(R(1) - v2);
+    R W;
+    if constexpr (kRecip<R>) W = rsq_(R(1) - v2);
+    else W = R(1) / rsqrt_(R(1) - v2);
     R h = R(1) + qdiv(gamma / (gamma - R(1)) * p, rmax(rho, C<R>::small));
     R w = rho * h;
     U[0] = rho * W;
@@ -341,7 +404,7 @@ AHD void hllc5(int n, const R* UL, const R* UR, const R* FL, const R* FR, R sL, 
     R s = left ? sL : sR, pK = left ? pL : pR, vK = left ? vL : vR;
     R den = s - sM + C<R>::small;
     R fac, dpx, dex;
-    if constexpr (sizeof(R) == 4) {
+    if constexpr (kRecip<R>) {
         const R rd = rcp_(den);
         fac = (s - vK) * rd;
         dpx = (pStar - pK) * rd;
@@ -425,7 +488,7 @@ AHD void r_p2c(const Phys<R>& P, const R* qin, R* U, R* rhoh_out = nullptr,
     R h = R(1) + qdiv(gamma / (gamma - R(1)) * p, rmax(rho, C<R>::small));
     R rhoh = rho * h;
     R vb = vx * Bx + vy * By + vz * Bz;
-    if constexpr (sizeof(R) == 4) {
+    if constexpr (kRecip<R>) {
         const R om = R(1) - (vx * vx + vy * vy + vz * vz);
         W = rsq_(om);
         const R iW = om * W;  // sqrt(1 - v^2)
@@ -515,7 +578,7 @@ template <typename R> AHD R r_fast_speed(const Phys<R>& P, const R* q) {
     R rhoh = rho * h;
     R vb = vx * Bx + vy * By + vz * Bz;
     R W, bx, by, bz;
-    if constexpr (sizeof(R) == 4) {
+    if constexpr (kRecip<R>) {
         W = rsq_(R(1) - v2);
         const R iW = (R(1) - v2) * W;
         const R b0 = W * vb;
@@ -674,6 +737,24 @@ AHD void r_face(const Phys<R>& P, int n, R* qL, R* qR, R* F, R& sL, R& sR) {
         if (!GIVEN) r_speeds(P, n, qL, qR, sL, sR);
     }
     r_riemann<RIEMANN, MUSCL_OVR>(P, n, qL, qR, UL, UR, FL, FR, sL, sR, F);
+}
+
+// The two states of a float64 (fd) RMHD face for callers that solve more than
+// one Riemann problem between them: floored primitives, conserved states,
+// fluxes and the face's own wave speeds, as r_face's float32 branch forms them.
+AHD void r_face_states(const Phys<fd>& P, int n, fd* qL, fd* qR, fd* UL, fd* UR, fd* FL, fd* FR,
+                       fd& sL, fd& sR) {
+    fd rhL, b2L, rhR, b2R, BBL, BBR, vbL, vbR, lmL, lpL, lmR, lpR;
+    floor_prim(P, qL);
+    floor_prim(P, qR);
+    r_p2c(P, qL, UL, &rhL, &b2L, &BBL, &vbL);
+    r_p2c(P, qR, UR, &rhR, &b2R, &BBR, &vbR);
+    r_flux_u(P, n, qL, UL, FL, BBL, vbL);
+    r_flux_u(P, n, qR, UR, FR, BBR, vbR);
+    eig_speeds(qL[1 + n], r_fast_speed_from(P, qL[4], rhL, b2L), lmL, lpL);
+    eig_speeds(qR[1 + n], r_fast_speed_from(P, qR[4], rhR, b2R), lmR, lpR);
+    sL = rmin(lmL, lmR);
+    sR = rmax(lpL, lpR);
 }
 
 // ------------------------------------------------------- con2prim (FP64) ---
