@@ -274,17 +274,27 @@ template <typename RF> __device__ __forceinline__ double ldf(const void* p, size
 }
 
 constexpr int kUpdateBlock = 128;
+enum { kC2PDefer = 0, kC2PFast = 1, kC2PReference = 2 };
 
-// DEFER: the learned con2prim runs in its own kernel, so this one only writes
-// U (the con2prim code is compiled out).  Every load is a plain coalesced
+// A counter of the whole warp (all 32 lanes), one atomic per warp.  One per thread
+// queues up at the counter's address at about one a clock: 0.6 M of them were
+// two thirds of a 1 M state con2prim batch.
+__device__ __forceinline__ void count_warp(unsigned long long* dst, unsigned n) {
+    n = __reduce_add_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0 && n) atomicAdd(dst, (unsigned long long)n);
+}
+
+// kC2PDefer: the con2prim runs in its own kernel, so this one only writes U (the
+// con2prim code is compiled out); kC2PFast / kC2PReference: r_c2p's two forms.  Every load is a plain coalesced
 // load with no dependence on an earlier one, so a thread's loads overlap each
 // other; 8 blocks of 128 threads per SM (64 registers, a few spilled) keep
 // more of them in flight than 6 blocks at 80 registers (3.81 against 3.96
 // ms/step; 10 and 12 blocks spill too much).  Staging the loads through
 // shared memory with per-thread cp.async streamed more slowly on B200 (4.2
 // against 6.4 TB/s for the same bytes).
-template <int PHYS, typename RF, bool DEFER, bool PASSIVE>
+template <int PHYS, typename RF, int C2P, bool PASSIVE>
 __global__ void __launch_bounds__(kUpdateBlock, PASSIVE ? 1 : 8) k_update(UpdArgs a) {
+    constexpr bool DEFER = C2P == kC2PDefer;
     constexpr int NM = PHYS == ASTRO_SRHD ? 5 : 9;
     constexpr int T = kUpdateBlock;
     const unsigned nc32 = (unsigned)a.nx * (unsigned)a.ny * (unsigned)a.nz;
@@ -317,32 +327,23 @@ __global__ void __launch_bounds__(kUpdateBlock, PASSIVE ? 1 : 8) k_update(UpdArg
             return ldf<RF>(d == 0 ? a.FxL : a.F[d], o);
         };
         double rhs[NM];
-        double rp[kMaxPassive];
+        double rp[PASSIVE ? kMaxPassive : 1];  // without passive fluxes: zero
 #pragma unroll
         for (int v = 0; v < NM; ++v) rhs[v] = 0.0;
-        for (int t = 0; t < np; ++t) rp[t] = 0.0;
+        if (PASSIVE)
+            for (int t = 0; t < np; ++t) rp[t] = 0.0;
         if (in) {
-            if constexpr (sizeof(RF) == 4) {
-                // float32 fluxes: multiply by 1/dx (the float64 path divides
-                // as the reference does)
-                const double i0 = a.idd[0], i1 = a.idd[1], i2 = a.idd[2];
+            // by 1/dx from the host: 27 float64 divisions per cell were most of
+            // the update's instructions (float64 RMHD, 78^3 cells: 72 us with
+            // them, 44 us without)
+            const double i0 = a.idd[0], i1 = a.idd[1], i2 = a.idd[2];
 #pragma unroll
-                for (int v = 0; v < NM; ++v) {
-                    double r = 0.0;
-                    r -= (flux(0, v, 1) - flux(0, v, 0)) * i0;
-                    r -= (flux(1, v, 1) - flux(1, v, 0)) * i1;
-                    r -= (flux(2, v, 1) - flux(2, v, 0)) * i2;
-                    rhs[v] = r;
-                }
-            } else {
-#pragma unroll
-                for (int v = 0; v < NM; ++v) {
-                    double r = 0.0;
-                    r -= (flux(0, v, 1) - flux(0, v, 0)) / a.dd[0];
-                    r -= (flux(1, v, 1) - flux(1, v, 0)) / a.dd[1];
-                    r -= (flux(2, v, 1) - flux(2, v, 0)) / a.dd[2];
-                    rhs[v] = r;
-                }
+            for (int v = 0; v < NM; ++v) {
+                double r = 0.0;
+                r -= (flux(0, v, 1) - flux(0, v, 0)) * i0;
+                r -= (flux(1, v, 1) - flux(1, v, 0)) * i1;
+                r -= (flux(2, v, 1) - flux(2, v, 0)) * i2;
+                rhs[v] = r;
             }
             if (PHYS == ASTRO_RMHD) {
                 const double* q = a.prk;
@@ -397,7 +398,7 @@ __global__ void __launch_bounds__(kUpdateBlock, PASSIVE ? 1 : 8) k_update(UpdArg
         if (a.rhs_only) {
 #pragma unroll
             for (int v = 0; v < NM; ++v) a.dst[(size_t)v * nc + cell] = rhs[v];
-            for (int t = 0; t < np; ++t) a.dst[(size_t)(NM + t) * nc + cell] = rp[t];
+            for (int t = 0; t < np; ++t) a.dst[(size_t)(NM + t) * nc + cell] = PASSIVE ? rp[t] : 0.0;
         } else {
             const Phys<double> P = Phys<double>::from(a.p);
             double q0[NM], U0[NM], Un[NM], q[NM];
@@ -429,7 +430,7 @@ __global__ void __launch_bounds__(kUpdateBlock, PASSIVE ? 1 : 8) k_update(UpdArg
             }
             if (!DEFER) {
                 if (PHYS == ASTRO_SRHD) s_c2p(P, Un, q);
-                else r_c2p(P, Un, q, cnt);
+                else r_c2p<C2P == kC2PFast>(P, Un, q, cnt);
 #pragma unroll
                 for (int v = 0; v < NM; ++v) a.dst[(size_t)v * nc + cell] = q[v];
                 if (a.dstf)
@@ -445,7 +446,7 @@ __global__ void __launch_bounds__(kUpdateBlock, PASSIVE ? 1 : 8) k_update(UpdArg
                     out = a.prk[(size_t)v * nc + cell];
                 } else if (np > 0 && t >= 0 && t < np) {
                     const size_t o = (size_t)v * nc + cell;
-                    const double t0 = a.pr0[o], r = rp[t];
+                    const double t0 = a.pr0[o], r = PASSIVE ? rp[t] : 0.0;
                     if (a.stage == 0) out = __dadd_rn(t0, __dmul_rn(dt, r));
                     else {
                         const double tk = a.prk[o];
@@ -463,17 +464,10 @@ __global__ void __launch_bounds__(kUpdateBlock, PASSIVE ? 1 : 8) k_update(UpdArg
         }
     }
     if (!DEFER && a.stats && !a.rhs_only) {
-        // warp-aggregated counters, one atomic per warp and counter
-        unsigned n1 = __reduce_add_sync(0xffffffffu, cell < nc ? 1u : 0u);
-        unsigned n2 = __reduce_add_sync(0xffffffffu, cnt.newton);
-        unsigned n3 = __reduce_add_sync(0xffffffffu, cnt.bisect);
-        unsigned n4 = __reduce_add_sync(0xffffffffu, cnt.hydro_fallback);
-        if ((threadIdx.x & 31) == 0) {
-            if (n1) atomicAdd(&a.stats->cells, (unsigned long long)n1);
-            if (n2) atomicAdd(&a.stats->newton, (unsigned long long)n2);
-            if (n3) atomicAdd(&a.stats->bisection, (unsigned long long)n3);
-            if (n4) atomicAdd(&a.stats->hydro_fallback, (unsigned long long)n4);
-        }
+        count_warp(&a.stats->cells, cell < nc ? 1u : 0u);
+        count_warp(&a.stats->newton, cnt.newton);
+        count_warp(&a.stats->bisection, cnt.bisect);
+        count_warp(&a.stats->hydro_fallback, cnt.hydro_fallback);
     }
 }
 
@@ -646,13 +640,15 @@ __global__ void __launch_bounds__(128, 5) k_c2p_learned(C2PArgs a) {
     }
     if (a.stats) {
         if (timed_out && t == 0) atomicAdd(&a.stats->wait_timeouts, 1ull);
-        atomicAdd(&a.stats->cells, (unsigned long long)n_cells);
-        if (n_polish) atomicAdd(&a.stats->learned_polish, (unsigned long long)n_polish);
-        if (n_fallback) atomicAdd(&a.stats->learned_fallback, (unsigned long long)n_fallback);
-        if (polish_steps) atomicAdd(&a.stats->polish_steps, (unsigned long long)polish_steps);
-        if (cnt.newton) atomicAdd(&a.stats->newton, (unsigned long long)cnt.newton);
-        if (cnt.bisect) atomicAdd(&a.stats->bisection, (unsigned long long)cnt.bisect);
-        if (cnt.hydro_fallback) atomicAdd(&a.stats->hydro_fallback, (unsigned long long)cnt.hydro_fallback);
+        count_warp(&a.stats->cells, n_cells);
+        count_warp(&a.stats->learned_polish, n_polish);
+        count_warp(&a.stats->learned_fallback, n_fallback);
+        count_warp(&a.stats->polish_steps, polish_steps);
+        if constexpr (!LISTED) {
+            count_warp(&a.stats->newton, cnt.newton);
+            count_warp(&a.stats->bisection, cnt.bisect);
+            count_warp(&a.stats->hydro_fallback, cnt.hydro_fallback);
+        }
     }
 }
 
@@ -675,9 +671,9 @@ __global__ void __launch_bounds__(128) k_c2p_fallback(C2PArgs a) {
             for (int v = 0; v < 9; ++v) a.qf[qf_index(a, (int)v, (long)cell)] = (float)q[v];
     }
     if (a.stats) {
-        if (cnt.newton) atomicAdd(&a.stats->newton, (unsigned long long)cnt.newton);
-        if (cnt.bisect) atomicAdd(&a.stats->bisection, (unsigned long long)cnt.bisect);
-        if (cnt.hydro_fallback) atomicAdd(&a.stats->hydro_fallback, (unsigned long long)cnt.hydro_fallback);
+        count_warp(&a.stats->newton, cnt.newton);
+        count_warp(&a.stats->bisection, cnt.bisect);
+        count_warp(&a.stats->hydro_fallback, cnt.hydro_fallback);
     }
 }
 
@@ -779,32 +775,31 @@ __global__ void k_prim_f32_rows(const double* __restrict__ pr, float* __restrict
 }
 
 // ------------------------------------------------------------- dispatch ---
-template <int PH, typename RF, bool DEF, bool PAS>
-void launch_update_t(const UpdArgs& a, dim3 grd, dim3 blk, cudaStream_t s) {
-    k_update<PH, RF, DEF, PAS><<<grd, blk, 0, s>>>(a);
+template <int PH, int C2P>
+void launch_update_t(const UpdArgs& a, dim3 grd, cudaStream_t s) {
+    const bool mixed = a.p.precision == ASTRO_PREC_MIXED;
+    if (passive_fluxes(a.p)) {
+        if (mixed) k_update<PH, float, C2P, true><<<grd, kUpdateBlock, 0, s>>>(a);
+        else k_update<PH, double, C2P, true><<<grd, kUpdateBlock, 0, s>>>(a);
+    } else {
+        if (mixed) k_update<PH, float, C2P, false><<<grd, kUpdateBlock, 0, s>>>(a);
+        else k_update<PH, double, C2P, false><<<grd, kUpdateBlock, 0, s>>>(a);
+    }
 }
+
+// r_c2p's operation order (see r_f_eval)
+inline bool c2p_fast(const AstroParams& p) { return p.recon != ASTRO_RECON_PPM; }
 
 cudaError_t launch_update(const UpdArgs& a, cudaStream_t s) {
     const size_t nc = (size_t)a.nx * a.ny * a.nz;
-    const dim3 blk(kUpdateBlock), grd((unsigned)((nc + kUpdateBlock - 1) / kUpdateBlock));
-    const bool mixed = a.p.precision == ASTRO_PREC_MIXED;
-    const bool pas = passive_fluxes(a.p);
-#define UPD(PH, DEF)                                                               \
-    do {                                                                           \
-        if (pas) {                                                                 \
-            if (mixed) launch_update_t<PH, float, DEF, true>(a, grd, blk, s);      \
-            else launch_update_t<PH, double, DEF, true>(a, grd, blk, s);           \
-        } else {                                                                   \
-            if (mixed) launch_update_t<PH, float, DEF, false>(a, grd, blk, s);     \
-            else launch_update_t<PH, double, DEF, false>(a, grd, blk, s);          \
-        }                                                                          \
-    } while (0)
+    const dim3 grd((unsigned)((nc + kUpdateBlock - 1) / kUpdateBlock));
+    // deferred: the learned path, and the GR steps' con2prim after the sources
     if (a.p.physics == ASTRO_SRHD) {
-        if (a.defer_c2p) UPD(ASTRO_SRHD, true);  // GR steps: con2prim after the sources
-        else UPD(ASTRO_SRHD, false);
-    } else if (a.defer_c2p) UPD(ASTRO_RMHD, true);
-    else UPD(ASTRO_RMHD, false);
-#undef UPD
+        if (a.defer_c2p) launch_update_t<ASTRO_SRHD, kC2PDefer>(a, grd, s);
+        else launch_update_t<ASTRO_SRHD, kC2PFast>(a, grd, s);
+    } else if (a.defer_c2p) launch_update_t<ASTRO_RMHD, kC2PDefer>(a, grd, s);
+    else if (c2p_fast(a.p)) launch_update_t<ASTRO_RMHD, kC2PFast>(a, grd, s);
+    else launch_update_t<ASTRO_RMHD, kC2PReference>(a, grd, s);
     mark(1, s);
     return cudaGetLastError();
 }
@@ -1117,32 +1112,47 @@ __global__ void k_p2c(AstroParams p, const double* q, double* U, long count) {
 
 // qf: optional float32 copy of the result in rows of `pitch` floats per nz
 // cells (the fused stages' input)
-__global__ void k_c2p(AstroParams p, const double* U, double* q, long count, AstroC2PStats* stats,
-                      float* qf = nullptr, int nz = 1, int pitch = 1) {
+template <int PHYS, bool FAST>
+__global__ void __launch_bounds__(128) k_c2p(AstroParams p, const double* U, double* q, long count,
+                                             AstroC2PStats* stats, float* qf, int nz, int pitch) {
+    constexpr int NM = PHYS == ASTRO_SRHD ? 5 : 9;
     const Phys<double> P = Phys<double>::from(p);
     C2PCount cnt;
     unsigned mine = 0;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < count;
          t += (long)gridDim.x * blockDim.x) {
-        double a[9], b[9];
-        const int nm = p.physics == ASTRO_SRHD ? 5 : 9;
-        for (int v = 0; v < nm; ++v) a[v] = U[(size_t)v * count + t];
-        if (p.physics == ASTRO_SRHD) s_c2p(P, a, b);
-        else r_c2p(P, a, b, cnt);
-        for (int v = 0; v < nm; ++v) q[(size_t)v * count + t] = b[v];
+        double a[NM], b[NM];
+#pragma unroll
+        for (int v = 0; v < NM; ++v) a[v] = U[(size_t)v * count + t];
+        if constexpr (PHYS == ASTRO_SRHD) s_c2p(P, a, b);
+        else r_c2p<FAST>(P, a, b, cnt);
+#pragma unroll
+        for (int v = 0; v < NM; ++v) q[(size_t)v * count + t] = b[v];
         if (qf) {
             const size_t rows = (size_t)(count / nz);
             const size_t r = (size_t)t / (unsigned)nz, k = (size_t)t % (unsigned)nz;
-            for (int v = 0; v < nm; ++v) qf[((size_t)v * rows + r) * pitch + k] = (float)b[v];
+#pragma unroll
+            for (int v = 0; v < NM; ++v) qf[((size_t)v * rows + r) * pitch + k] = (float)b[v];
         }
         ++mine;
     }
     if (stats) {
-        atomicAdd(&stats->cells, (unsigned long long)mine);
-        if (cnt.newton) atomicAdd(&stats->newton, (unsigned long long)cnt.newton);
-        if (cnt.bisect) atomicAdd(&stats->bisection, (unsigned long long)cnt.bisect);
-        if (cnt.hydro_fallback) atomicAdd(&stats->hydro_fallback, (unsigned long long)cnt.hydro_fallback);
+        count_warp(&stats->cells, mine);
+        count_warp(&stats->newton, cnt.newton);
+        count_warp(&stats->bisection, cnt.bisect);
+        count_warp(&stats->hydro_fallback, cnt.hydro_fallback);
     }
+}
+
+void launch_c2p(const AstroParams& p, bool fast, const double* U, double* q, long count,
+                AstroC2PStats* stats, int grid, cudaStream_t s, float* qf = nullptr, int nz = 1,
+                int pitch = 1) {
+    if (p.physics == ASTRO_SRHD)
+        k_c2p<ASTRO_SRHD, true><<<grid, 128, 0, s>>>(p, U, q, count, stats, qf, nz, pitch);
+    else if (fast)
+        k_c2p<ASTRO_RMHD, true><<<grid, 128, 0, s>>>(p, U, q, count, stats, qf, nz, pitch);
+    else
+        k_c2p<ASTRO_RMHD, false><<<grid, 128, 0, s>>>(p, U, q, count, stats, qf, nz, pitch);
 }
 
 // ------------------------------------------------------------ sources ---
@@ -1695,8 +1705,7 @@ static int run_stage_fused(const AstroParams* p, const AstroGrid* g, const Layou
         c.qf = dstf; c.qf_nz = g->nz; c.qf_pitch = L.pitch;
         e = launch_c2p_learned(c, s);
     } else {
-        k_c2p<<<sm_count_cached() * 8, 128, 0, s>>>(*p, U, dst, (long)nc, stats, dstf, g->nz,
-                                                    L.pitch);
+        launch_c2p(*p, c2p_fast(*p), U, dst, (long)nc, stats, grid_for(nc, 128), s, dstf, g->nz, L.pitch);
         mark(1, s);
         e = cudaGetLastError();
     }
@@ -1934,7 +1943,7 @@ int astro_c2p(const AstroParams* p, const double* cons, double* prim, int64_t co
     if (!p || count < 0) return ASTRO_E_INVALID;
     if (count == 0) return ASTRO_OK;  // an empty batch may pass null arrays
     if (!prim || !cons) return ASTRO_E_INVALID;
-    k_c2p<<<grid_for(count, 128), 128, 0, (cudaStream_t)stream>>>(*p, cons, prim, count, stats);
+    launch_c2p(*p, true, cons, prim, count, stats, grid_for(count, 128), (cudaStream_t)stream);
     mark(2, (cudaStream_t)stream);
     return cuda_status(cudaGetLastError());
 }
@@ -2119,7 +2128,7 @@ int astro_step_gr(const AstroParams* p, const AstroGrid* g, const AstroGR* gr,
             c.fb_cap = (unsigned)c2p_fb_capacity(*g);
             e = launch_c2p_learned(c, s);
         } else {
-            k_c2p<<<sm_count_cached() * 8, 128, 0, s>>>(*p, U, dst, (long)nc, stats);
+            launch_c2p(*p, c2p_fast(*p), U, dst, (long)nc, stats, grid_for(nc, 128), s);
             mark(2, s);
             e = cudaGetLastError();
         }

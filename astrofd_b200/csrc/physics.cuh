@@ -865,11 +865,14 @@ AHD double r_f_of_Z(const Phys<double>& P, double Z, double D, double tau, doubl
     return tau_calc - tau;
 }
 
-// f(Z) in the reference's operation order (float64 reference mode), or
-// (FAST) the same expressions with the divisions regrouped (r_f_df_of_Z):
-// equal to rounding, with a dependency chain about half as long, for the
-// learned path's fallback solves, whose time is the latency of its slowest
-// cells
+// f(Z) with the divisions regrouped (FAST, r_f_df_of_Z: a third of the float64
+// operations, a dependency chain half as long) or in the reference's operation
+// order; equal to rounding.  The reference's order is kept for PPM blocks, whose
+// flattening test compares neighbouring cells: in the cells outside the updated
+// range, which every stage converts to and fro, pressures that began equal differ
+// by the conversion's rounding alone, and its sign then switches a face value by
+// their difference to the next updated cell.  (RMHD 134^3 cells, per stage: the
+// update takes 300 us with the regrouped form, 425 us with the reference's.)
 template <bool FAST>
 AHD double r_f_eval(const Phys<double>& P, double Z, double D, double tau, double B2,
                     double SB, double S2) {
@@ -880,16 +883,13 @@ AHD double r_f_eval(const Phys<double>& P, double Z, double D, double tau, doubl
 // The reference's Newton on Z from a starting value: up to 50 steps with the
 // forward-difference derivative and +-Z/2 step clamp (rmhd_core.py:268-292).
 // Returns true when |f| < 1e-10 max(1, tau).
-template <bool FAST = false>
+template <bool FAST>
 AHD bool r_newton(const Phys<double>& P, double& Z, int max_it, double D, double tau,
-                  double B2, double SB, double S2, int* steps = nullptr) {
+                  double B2, double SB, double S2) {
     const double tol = 1e-10 * rmax(1.0, tau);
     for (int it = 0; it < max_it; ++it) {
         double f = r_f_eval<FAST>(P, Z, D, tau, B2, SB, S2);
-        if (fabs(f) < tol) {
-            if (steps) *steps = it;
-            return true;
-        }
+        if (fabs(f) < tol) return true;
         double eps = 1e-6 * rmax(1.0, Z);
         double fp = r_f_eval<FAST>(P, Z + eps, D, tau, B2, SB, S2);
         double dfdZ = (fp - f) / eps;
@@ -900,13 +900,12 @@ AHD bool r_newton(const Phys<double>& P, double& Z, int max_it, double D, double
         Z += dZ;
         if (Z < 1e-12) Z = 1e-12;
     }
-    if (steps) *steps = max_it;
     return false;
 }
 
 // Primitive recovery once Z is known (rmhd_core.py:320-341); FAST as in
 // r_f_eval
-template <bool FAST = false>
+template <bool FAST>
 AHD void r_prims_from_Z(const Phys<double>& P, double Z, const double* U, const double* q0,
                         double* q, C2PCount& cnt) {
     const double G = P.gamma, SM = 1e-12;
@@ -955,7 +954,7 @@ AHD void r_prims_from_Z(const Phys<double>& P, double Z, const double* U, const 
 }
 
 // Bisection fallback (rmhd_core.py:294-318); Z holds the last Newton iterate
-template <bool FAST = false>
+template <bool FAST>
 AHD void r_bisect(const Phys<double>& P, double& Z, double Z1, double D, double tau, double B2,
                   double SB, double S2) {
     double Zmin = 1e-12;
@@ -1181,10 +1180,9 @@ AHD bool r_prims_from_Z_checked(const Phys<double>& P, double Z, const double* U
     return true;
 }
 
-// Full reference con2prim (cons_to_prim_rmhd, rmhd_core.py:249-341); FAST:
-// its f(Z) and primitive recovery with the regrouped divisions (the learned
-// path's fallback), otherwise the reference's operation order
-template <bool FAST = false>
+// Full reference con2prim (cons_to_prim_rmhd, rmhd_core.py:249-341); FAST as in
+// r_f_eval
+template <bool FAST>
 AHD void r_c2p(const Phys<double>& P, const double* U, double* q, C2PCount& cnt) {
     double D = U[0], tau = U[4];
     double B2 = U[5] * U[5] + U[6] * U[6] + U[7] * U[7];
