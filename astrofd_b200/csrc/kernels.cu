@@ -285,13 +285,15 @@ __device__ __forceinline__ void count_warp(unsigned long long* dst, unsigned n) 
 }
 
 // kC2PDefer: the con2prim runs in its own kernel, so this one only writes U (the
-// con2prim code is compiled out); kC2PFast / kC2PReference: r_c2p's two forms.  Every load is a plain coalesced
-// load with no dependence on an earlier one, so a thread's loads overlap each
-// other; 8 blocks of 128 threads per SM (64 registers, a few spilled) keep
-// more of them in flight than 6 blocks at 80 registers (3.81 against 3.96
-// ms/step; 10 and 12 blocks spill too much).  Staging the loads through
-// shared memory with per-thread cp.async streamed more slowly on B200 (4.2
-// against 6.4 TB/s for the same bytes).
+// con2prim code is compiled out); kC2PFast / kC2PReference: r_c2p's two forms.
+// Every load is a plain coalesced load with no dependence on an earlier one, so a
+// thread's loads overlap each other; 8 blocks of 128 threads per SM (64 registers,
+// a few spilled) keep more of them in flight than 6 blocks at 80 registers (3.81
+// against 3.96 ms/step; 10 and 12 blocks spill too much).  Staging the loads
+// through shared memory with per-thread cp.async streamed more slowly on B200 (4.2
+// against 6.4 TB/s for the same bytes), and in one kernel with the learned con2prim
+// (U in registers, 20 warps per SM beside its shared memory) the two took 3.64 ms
+// per 262^3 stage against 2.54 ms apart.
 template <int PHYS, typename RF, int C2P, bool PASSIVE>
 __global__ void __launch_bounds__(kUpdateBlock, PASSIVE ? 1 : 8) k_update(UpdArgs a) {
     constexpr bool DEFER = C2P == kC2PDefer;
@@ -787,8 +789,12 @@ void launch_update_t(const UpdArgs& a, dim3 grd, cudaStream_t s) {
     }
 }
 
-// r_c2p's operation order (see r_f_eval)
-inline bool c2p_fast(const AstroParams& p) { return p.recon != ASTRO_RECON_PPM; }
+// r_c2p's operation order (see r_f_eval): regrouped where nothing after it turns
+// its rounding into a jump, as PPM's flattening test does, and the float32 copy of
+// the mixed path (a last-bit change of a float32 velocity at W = 10 is 1e-5 of W^2)
+inline bool c2p_fast(const AstroParams& p) {
+    return p.recon != ASTRO_RECON_PPM && p.precision == ASTRO_PREC_FP64;
+}
 
 cudaError_t launch_update(const UpdArgs& a, cudaStream_t s) {
     const size_t nc = (size_t)a.nx * a.ny * a.nz;
