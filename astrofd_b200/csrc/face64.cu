@@ -24,7 +24,7 @@
 // Bound: the float64 pipe (about 850 float64 operations per RMHD WENO5 face) at 16
 // warps per SM, 128 registers.  One stage's faces of 134^3 cells, RMHD WENO5 "hlld"
 // with carried x faces: 2204 us as four per-face passes with IEEE divisions, 636 us
-// here; SRHD PPM HLLC 377 us, 241 us.  (3 blocks per SM, which spill nothing: 659 and
+// here; SRHD PPM HLLC 377 us, 228 us.  (3 blocks per SM, which spill nothing: 659 and
 // 276 us.)
 #include "face64.cuh"
 
@@ -234,8 +234,11 @@ __device__ __forceinline__ void walk(const Args& a, double* sh, unsigned block) 
                                                  wide);
 }
 
+// Blocks per SM: SRHD 8 (64 registers: 4 blocks at 128 take 723 against 683 us for
+// a 128^3 PPM step's faces, 113 against 89 us for a 64^3 MUSCL one's); RMHD 4 (128
+// registers); "hlld_full" 2.
 template <int PHYS, int RECON, int RIEMANN>
-__global__ void __launch_bounds__(T, RIEMANN == ASTRO_RIEMANN_HLLD_FULL ? 2 : 4)
+__global__ void __launch_bounds__(T, PHYS == ASTRO_SRHD ? 8 : (RIEMANN == ASTRO_RIEMANN_HLLD_FULL ? 2 : 4))
     k_face64(const __grid_constant__ Args a) {
     constexpr int NM = PHYS == ASTRO_SRHD ? 5 : 9;
     __shared__ double sh[NM * T];
