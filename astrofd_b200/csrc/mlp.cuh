@@ -12,6 +12,7 @@
 //   forward      H_l[128 x out] = H_{l-1}[128 x in] . W_l^T           (A, B K-major)
 //   data grad    dH_{l-1}[128 x in] = dZ_l[128 x out] . W_l           (A K-major, B MN-major)
 //   weight grad  dW_l[out(pad 128) x in] = dZ_l^T . H_{l-1}           (A, B MN-major)
+//   bias grad    db_l[out(pad 128)] = dZ_l^T . 1 (16 columns of ones) (A, B MN-major)
 // Operands use the SWIZZLE_NONE canonical layout: 8x8 core matrices of 8
 // rows x 16 bytes; element (r, c) of an R-row operand lives at byte
 //   (c/8)*(R/8)*128 + (r/8)*128 + (r%8)*16 + (c%8)*2,
@@ -53,8 +54,8 @@ constexpr int OFF_DZ = OFF_H3 + 128 * 64 * 2;  // [128 x 128] bf16, 32 KB (16 co
 constexpr int OFF_DS1 = OFF_DZ + 128 * 128 * 2;  // ReLU'(z) of layers 1..3, bf16 16 KB each
 constexpr int OFF_DS2 = OFF_DS1 + 128 * 64 * 2;
 constexpr int OFF_DS3 = OFF_DS2 + 128 * 64 * 2;
-constexpr int OFF_RED = OFF_DS3 + 128 * 64 * 2;  // [128][65] f32 bias-gradient reduction
-constexpr int OFF_BAR = OFF_RED + 128 * 65 * 4;  // mbarrier (8 B) + TMEM address (4 B)
+constexpr int OFF_ONE = OFF_DS3 + 128 * 64 * 2;  // [128 x 16] bf16 ones: bias gradients
+constexpr int OFF_BAR = OFF_ONE + 128 * 16 * 2;  // mbarrier (8 B) + TMEM address (4 B)
 constexpr int kTrainSmem = OFF_BAR + 16;
 static_assert(kTrainSmem <= 227 * 1024, "training tile exceeds shared memory");
 
@@ -244,28 +245,52 @@ __device__ __forceinline__ void st_row8_packed(unsigned char* base, int R, int r
     *reinterpret_cast<uint4*>(base + elem_off(R, r, c0)) = make_uint4(p[0], p[1], p[2], p[3]);
 }
 
+// 8 consecutive float32 weights as bfloat16 into columns [c, c + 8) of row o
+__device__ __forceinline__ void put_row8(unsigned char* base, int R, int o, int c, float4 a, float4 b) {
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    st_row8(base, R, o, c, v);
+}
+
 // FP32 master weights -> bf16 K-major operands in shared memory (all
-// threads), biases in float32.
+// threads), biases in float32.  Sixteen-byte loads of eight weights at a time, all
+// of a thread's in flight together: weight by weight this was 6 us of every
+// block's start.
 __device__ __forceinline__ void load_weights(unsigned char* sm, const Params* P) {
-    for (int e = threadIdx.x; e < 64 * 16; e += blockDim.x) {  // W1 [64 x 16], in 5..15 = 0
-        int o = e / 16, i = e % 16;
-        float w = i < NIN ? P->W1[o * NIN + i] : 0.f;
-        *reinterpret_cast<__nv_bfloat16*>(sm + OFF_W1 + elem_off(64, o, i)) = __float2bfloat16_rn(w);
+    const bool wide = (reinterpret_cast<uintptr_t>(P) & 15) == 0;
+    auto row8 = [&](const float* w, float4& a, float4& b) {
+        if (wide) {
+            a = reinterpret_cast<const float4*>(w)[0];
+            b = reinterpret_cast<const float4*>(w)[1];
+        } else {
+            a = make_float4(w[0], w[1], w[2], w[3]);
+            b = make_float4(w[4], w[5], w[6], w[7]);
+        }
+    };
+    // W2, W3 [64 x 64]: 512 groups of eight each
+#pragma unroll 4
+    for (int e = threadIdx.x; e < 512; e += TILE) {
+        const int o = e >> 3, c = (e & 7) * 8;
+        float4 a, b, x, y;
+        row8(P->W2 + o * H + c, a, b);
+        row8(P->W3 + o * H + c, x, y);
+        put_row8(sm + OFF_W2, 64, o, c, a, b);
+        put_row8(sm + OFF_W3, 64, o, c, x, y);
     }
-    for (int e = threadIdx.x; e < 64 * 64; e += blockDim.x) {
-        int o = e / 64, i = e % 64;
-        *reinterpret_cast<__nv_bfloat16*>(sm + OFF_W2 + elem_off(64, o, i)) =
-            __float2bfloat16_rn(P->W2[o * H + i]);
-        *reinterpret_cast<__nv_bfloat16*>(sm + OFF_W3 + elem_off(64, o, i)) =
-            __float2bfloat16_rn(P->W3[o * H + i]);
+    {   // W4 [16 x 64], rows 2..15 = 0: 128 groups
+        const int e = threadIdx.x, o = e >> 3, c = (e & 7) * 8;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (o < NOUT) row8(P->W4 + o * H + c, a, b);
+        put_row8(sm + OFF_W4, 16, o, c, a, b);
     }
-    for (int e = threadIdx.x; e < 16 * 64; e += blockDim.x) {  // W4 [16 x 64], rows 2..15 = 0
-        int o = e / 64, i = e % 64;
-        float w = o < NOUT ? P->W4[o * H + i] : 0.f;
-        *reinterpret_cast<__nv_bfloat16*>(sm + OFF_W4 + elem_off(16, o, i)) = __float2bfloat16_rn(w);
+    {   // W1 [64 x 16], inputs 5..15 = 0: 128 groups
+        const int e = threadIdx.x, o = e >> 1, c = (e & 1) * 8;
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = c + i < NIN ? P->W1[o * NIN + c + i] : 0.f;
+        st_row8(sm + OFF_W1, 64, o, c, v);
     }
     float* bs = reinterpret_cast<float*>(sm + OFF_BIAS);
-    for (int e = threadIdx.x; e < 3 * H + NOUT; e += blockDim.x)
+    for (int e = threadIdx.x; e < 3 * H + NOUT; e += TILE)
         bs[e] = e < H ? P->b1[e]
                       : (e < 2 * H ? P->b2[e - H] : (e < 3 * H ? P->b3[e - 2 * H] : P->b4[e - 3 * H]));
 }
