@@ -23,9 +23,9 @@
 //
 // Bound: the float64 pipe (about 850 float64 operations per RMHD WENO5 face) at 16
 // warps per SM, 128 registers.  One stage's faces of 134^3 cells, RMHD WENO5 "hlld"
-// with carried x faces: 2204 us as four per-face passes with IEEE divisions, 636 us
-// here; SRHD PPM HLLC 377 us, 228 us.  (3 blocks per SM, which spill nothing: 659 and
-// 276 us.)
+// with carried x faces: 2204 us as four per-face passes with IEEE divisions, 631 us
+// here; SRHD PPM HLLC 377 us, 220 us.  (RMHD at 3 blocks per SM, which spill nothing,
+// 4 % slower; at 5, 1 %.)
 #include "face64.cuh"
 
 #include <stdint.h>
@@ -242,11 +242,16 @@ __global__ void __launch_bounds__(T, PHYS == ASTRO_SRHD ? 8 : (RIEMANN == ASTRO_
     k_face64(const __grid_constant__ Args a) {
     constexpr int NM = PHYS == ASTRO_SRHD ? 5 : 9;
     __shared__ double sh[NM * T];
-    if (blockIdx.x < (unsigned)a.blocks_z) {
+    // the walks first: the short z blocks then fill the launch's end
+    if (blockIdx.x < (unsigned)a.blocks_x) {
+        walk<PHYS, RECON, RIEMANN, 0>(a, sh, blockIdx.x);
+    } else if (blockIdx.x < (unsigned)(a.blocks_x + a.blocks_y)) {
+        walk<PHYS, RECON, RIEMANN, 1>(a, sh, blockIdx.x - a.blocks_x);
+    } else {
         // one warp per 31 z faces of a row: lane 0 only makes left states
         const int lo = a.b.lo, faces = a.b.hi[2] - lo + 1;
         const unsigned per = (unsigned)(faces + 30) / 31;
-        const unsigned wp = blockIdx.x * (T / 32) + threadIdx.x / 32;
+        const unsigned wp = (blockIdx.x - a.blocks_x - a.blocks_y) * (T / 32) + threadIdx.x / 32;
         const unsigned r = wp / per, ey = (unsigned)(a.b.hi[1] - lo);
         const int i = lo + (int)(r / ey), j = lo + (int)(r % ey);
         if (i >= a.b.hi[0]) return;
@@ -255,10 +260,6 @@ __global__ void __launch_bounds__(T, PHYS == ASTRO_SRHD ? 8 : (RIEMANN == ASTRO_
         bool wide = false;
         cell_and_face<PHYS, RECON, RIEMANN, 2>(a, sh, i, j, k < a.b.hi[2] ? k : a.b.hi[2],
                                                (threadIdx.x & 31) > 0 && k <= a.b.hi[2], wide);
-    } else if (blockIdx.x < (unsigned)(a.blocks_z + a.blocks_y)) {
-        walk<PHYS, RECON, RIEMANN, 1>(a, sh, blockIdx.x - a.blocks_z);
-    } else {
-        walk<PHYS, RECON, RIEMANN, 0>(a, sh, blockIdx.x - a.blocks_z - a.blocks_y);
     }
 }
 
@@ -276,20 +277,40 @@ cudaError_t launch(Args a, int sms, cudaStream_t s) {
     if (e[0] <= 0 || e[1] <= 0 || e[2] <= 0) return cudaSuccess;
     long blocks[3] = {0, 0, 0};
     if (a.F[2]) blocks[2] = (e[0] * e[1] * ((e[2] + 1 + 30) / 31) + T / 32 - 1) / (T / 32);
+    const long resident =
+        (long)sms * (a.p.physics == ASTRO_SRHD ? 8 : (a.p.riemann == ASTRO_RIEMANN_HLLD_FULL ? 2 : 4));
     for (int d = 0; d < 2; ++d) {
         if (!a.F[d]) continue;
-        // A longer walk repeats fewer reconstructions at its start (1 per
-        // segment); a shorter one gives more threads.  Four times the resident
-        // threads (4 blocks per SM) keep the last wave small; up to 16 faces per
-        // thread, where the repeated share is 6 %.
-        const long plane = e[1 - d] * e[2], faces = e[d] + 1;
-        long seg = plane * faces / ((long)sms * 4 * T * 4);
-        if (seg < 1) seg = 1;
-        if (seg > 16) seg = 16;
-        a.seg[d] = (int)seg;
-        blocks[d] = ((plane + T - 1) / T) * ((faces + seg - 1) / seg);
+        // A longer walk repeats fewer reconstructions at its start (about 0.6 of a
+        // turn per segment); more segments give more blocks.  With z blocks behind
+        // them the walks are as long as leaves one block for each place on the
+        // device, up to 16 faces; alone, of the lengths up to 32 the one that needs
+        // the fewest turns with whole waves of blocks (128^3 RMHD x faces: 129 as 9
+        // segments of 15 are 2 waves, as 19 of 7 they were 5).  Segments of equal
+        // length.  Against 4 waves of walks with z first: ragged 90 x 61 x 103 PPM
+        // faces 174 -> 151 us, Kerr-Schild 72^3 WENO5 163 -> 136 us per stage, SRHD
+        // 128^3 PPM 228 -> 220 us.
+        const long per = (e[1 - d] * e[2] + T - 1) / T, faces = e[d] + 1;
+        long seg = 1;
+        if (a.F[2]) {
+            seg = per * faces / resident;
+            seg = seg < 1 ? 1 : (seg > 16 ? 16 : seg);
+        } else {
+            double best = 0.0;
+            for (long s = 1; s <= 32 && s <= faces; ++s) {
+                const long n = per * ((faces + s - 1) / s);
+                const double cost = (double)((n + resident - 1) / resident) * ((double)s + 0.6);
+                if (s == 1 || cost < best) {
+                    best = cost;
+                    seg = s;
+                }
+            }
+        }
+        const long nseg = (faces + seg - 1) / seg;
+        a.seg[d] = (int)((faces + nseg - 1) / nseg);
+        blocks[d] = per * ((faces + a.seg[d] - 1) / a.seg[d]);
     }
-    a.blocks_z = (int)blocks[2];
+    a.blocks_x = (int)blocks[0];
     a.blocks_y = (int)blocks[1];
     const long total = blocks[0] + blocks[1] + blocks[2];
     if (total == 0) return cudaSuccess;

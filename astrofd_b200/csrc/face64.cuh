@@ -17,8 +17,8 @@ struct Args {
     const double* carried;  // those speeds (an earlier launch's speeds_out)
     int ndiss;
     AstroParams p;
-    // set by launch(): thread blocks of z, y (x follow) and faces per thread
-    int blocks_z, blocks_y, seg[2];
+    // set by launch(): thread blocks of x, y (z follow) and faces per thread
+    int blocks_x, blocks_y, seg[2];
 };
 
 cudaError_t launch(Args a, int sms, cudaStream_t s);

@@ -655,8 +655,11 @@ __global__ void __launch_bounds__(128, 5) k_c2p_learned(C2PArgs a) {
 }
 
 // The cells k_c2p_learned listed: the reference's complete con2prim, one cell
-// per thread.
-__global__ void __launch_bounds__(128) k_c2p_fallback(C2PArgs a) {
+// per thread.  Bound by its chains of dependent float64 operations, so as many warps
+// as fit without spilling: 6 blocks per SM at 80 registers (1.4 M cells 175 us at 4
+// blocks, 158 at 5, 150 at 6, 192 at 8, which spill).
+constexpr int kFallbackBlocks = 6;
+__global__ void __launch_bounds__(128, kFallbackBlocks) k_c2p_fallback(C2PArgs a) {
     const unsigned n = min(*a.fb_count, a.fb_cap);
     const Phys<double> P = Phys<double>::from(a.p);
     C2PCount cnt;
@@ -742,7 +745,7 @@ cudaError_t launch_c2p_learned_t(const C2PArgs& a, cudaStream_t s) {
     k_c2p_learned<LISTED><<<grid, mlp::TILE, mlp::kInferSmem + 16, s>>>(a);
     mark(3, s);
     if (LISTED) {
-        k_c2p_fallback<<<sm_count_cached() * 4, 128, 0, s>>>(a);
+        k_c2p_fallback<<<sm_count_cached() * kFallbackBlocks, 128, 0, s>>>(a);
         mark(4, s);
     }
     return cudaGetLastError();
