@@ -55,7 +55,7 @@ __device__ __forceinline__ bool face_stored_finite(const FaceArgs& a, size_t nc,
 // the list is incomplete: every face of the pass is then checked and the
 // non-finite ones are recomputed, so no float32 failure is left in place.
 template <int PHYS, int RECON, int RIEMANN, bool GIVEN, int DIR>
-__global__ void __launch_bounds__(128) k_face_fix(FaceArgs a) {
+__device__ __forceinline__ void fix_pass(const FaceArgs& a) {
     constexpr int NM = PHYS == ASTRO_SRHD ? 5 : 9;
     const unsigned cnt = *a.fix_count;
     if (cnt <= a.fix_cap) {
@@ -86,64 +86,119 @@ __global__ void __launch_bounds__(128) k_face_fix(FaceArgs a) {
     }
 }
 
-// direction is a template parameter so the per-direction component indices
-// fold to constants and the face state stays in registers
-template <int PH, int RE, int RI>
-cudaError_t launch_face_dir(const FaceArgs& a, bool given, dim3 grd, dim3 blk, cudaStream_t s) {
-    const dim3 fgrd(148 * 4);
-    // the fix-up counter starts every pass at zero (the workspace, or the
-    // shared static scratch, holds the previous pass's count)
-    const cudaError_t e = cudaMemsetAsync(a.fix_count, 0, sizeof(unsigned), s);
-    if (e != cudaSuccess) return e;
-    if constexpr (PH == ASTRO_RMHD && RE != ASTRO_RECON_MUSCL) {
+template <int PHYS, int RECON, int RIEMANN, bool GIVEN, int DIR>
+__global__ void __launch_bounds__(128) k_face_fix(const __grid_constant__ FaceArgs a) {
+    fix_pass<PHYS, RECON, RIEMANN, GIVEN, DIR>(a);
+}
+
+// all three directions' lists in one launch (blockIdx.y)
+struct FaceArgs3 {
+    FaceArgs d[3];
+};
+template <int PHYS, int RECON, int RIEMANN>
+__global__ void __launch_bounds__(128) k_face_fix3(const __grid_constant__ FaceArgs3 a) {
+    if (blockIdx.y == 0) fix_pass<PHYS, RECON, RIEMANN, false, 0>(a.d[0]);
+    else if (blockIdx.y == 1) fix_pass<PHYS, RECON, RIEMANN, false, 1>(a.d[1]);
+    else fix_pass<PHYS, RECON, RIEMANN, false, 2>(a.d[2]);
+}
+
+dim3 face_grid(const FaceArgs& a) {
+    const unsigned plane = (unsigned)a.ext[1] * (unsigned)a.ext[2];
+    return dim3((plane + 127) / 128, (unsigned)(a.ext[0] < 65535 ? a.ext[0] : 65535));
+}
+
+// an empty cell range in any direction: no faces (checked per extent, since two
+// negative extents would give a positive product)
+bool empty(const FaceArgs& a) { return a.ext[0] <= 0 || a.ext[1] <= 0 || a.ext[2] <= 0; }
+
+// The fix-up counters start every pass at zero (the workspace, or the shared
+// static scratch, holds the previous pass's count).
+//
+// one direction and its listed faces, for the carried order of passes
+template <int RE, int RI>
+struct OnePass {
+    static cudaError_t run(const FaceArgs& a, bool given, cudaStream_t s) {
+        constexpr int PH = ASTRO_RMHD;
+        const dim3 fgrd(148 * 4), grd = face_grid(a);
+        const cudaError_t e = cudaMemsetAsync(a.fix_count, 0, sizeof(unsigned), s);
+        if (e != cudaSuccess) return e;
         if (given) {
-            k_face<PH, RE, RI, true, 0><<<grd, blk, 0, s>>>(a);
-            k_face_fix<PH, RE, RI, true, 0><<<fgrd, blk, 0, s>>>(a);
-            return cudaSuccess;
+            k_face<PH, RE, RI, true, 0><<<grd, 128, 0, s>>>(a);
+            k_face_fix<PH, RE, RI, true, 0><<<fgrd, 128, 0, s>>>(a);
+        } else if (a.dir == 0) {
+            k_face<PH, RE, RI, false, 0><<<grd, 128, 0, s>>>(a);
+            k_face_fix<PH, RE, RI, false, 0><<<fgrd, 128, 0, s>>>(a);
+        } else if (a.dir == 1) {
+            k_face<PH, RE, RI, false, 1><<<grd, 128, 0, s>>>(a);
+            k_face_fix<PH, RE, RI, false, 1><<<fgrd, 128, 0, s>>>(a);
+        } else {
+            k_face<PH, RE, RI, false, 2><<<grd, 128, 0, s>>>(a);
+            k_face_fix<PH, RE, RI, false, 2><<<fgrd, 128, 0, s>>>(a);
         }
+        return cudaGetLastError();
     }
-    if (a.dir == 0) {
-        k_face<PH, RE, RI, false, 0><<<grd, blk, 0, s>>>(a);
-        k_face_fix<PH, RE, RI, false, 0><<<fgrd, blk, 0, s>>>(a);
-    } else if (a.dir == 1) {
-        k_face<PH, RE, RI, false, 1><<<grd, blk, 0, s>>>(a);
-        k_face_fix<PH, RE, RI, false, 1><<<fgrd, blk, 0, s>>>(a);
-    } else {
-        k_face<PH, RE, RI, false, 2><<<grd, blk, 0, s>>>(a);
-        k_face_fix<PH, RE, RI, false, 2><<<fgrd, blk, 0, s>>>(a);
+};
+
+// The three directions are independent: their listed faces are recomputed by one
+// launch behind them and one clear precedes them, 5 launches instead of 9
+// (SSPRK3 step of a 75 x 130 x 121 slab 1314 -> 1276 us).
+template <int PH, int RE, int RI>
+cudaError_t run_all(const FaceArgs3& a, void (*launched)(cudaStream_t), cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(a.d[0].fix_count, 0, 3 * sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    if (!empty(a.d[2])) {
+        k_face<PH, RE, RI, false, 2><<<face_grid(a.d[2]), 128, 0, s>>>(a.d[2]);
+        launched(s);
     }
-    return cudaSuccess;
+    if (!empty(a.d[0])) {
+        k_face<PH, RE, RI, false, 0><<<face_grid(a.d[0]), 128, 0, s>>>(a.d[0]);
+        launched(s);
+    }
+    if (!empty(a.d[1])) k_face<PH, RE, RI, false, 1><<<face_grid(a.d[1]), 128, 0, s>>>(a.d[1]);
+    k_face_fix3<PH, RE, RI><<<dim3(148, 3), 128, 0, s>>>(a);
+    launched(s);
+    return cudaGetLastError();
+}
+
+template <int PH, int RE>
+cudaError_t run_riemann(const FaceArgs3& a, void (*launched)(cudaStream_t), cudaStream_t s) {
+    const int ri = a.d[0].p.riemann;
+    if constexpr (PH == ASTRO_RMHD)
+        if (ri == 2) return run_all<PH, RE, 2>(a, launched, s);
+    return ri == 1 ? run_all<PH, RE, 1>(a, launched, s) : run_all<PH, RE, 0>(a, launched, s);
 }
 
 }  // namespace
 
-cudaError_t launch(const FaceArgs& a, bool given, cudaStream_t s) {
-    // an empty cell range in any direction: no faces (checked per extent,
-    // since two negative extents would give a positive product)
-    if (a.ext[0] <= 0 || a.ext[1] <= 0 || a.ext[2] <= 0) return cudaSuccess;
-    const unsigned plane = (unsigned)a.ext[1] * (unsigned)a.ext[2];
-    const dim3 blk(128), grd((plane + 127) / 128, (unsigned)(a.ext[0] < 65535 ? a.ext[0] : 65535));
-    const AstroParams& p = a.p;
-    cudaError_t me = cudaSuccess;
-#define FACE(PH, RE, RI) me = launch_face_dir<PH, RE, RI>(a, given, grd, blk, s)
-#define RECONS(PH, RI)                                                          \
-    do {                                                                        \
-        if (p.recon == 0) FACE(PH, 0, RI);                                      \
-        else if (p.recon == 1) FACE(PH, 1, RI);                                 \
-        else FACE(PH, 2, RI);                                                   \
-    } while (0)
-    if (p.physics == ASTRO_SRHD) {
-        if (p.riemann == 1) RECONS(ASTRO_SRHD, 1);
-        else RECONS(ASTRO_SRHD, 0);
-    } else {
-        if (p.riemann == 2) RECONS(ASTRO_RMHD, 2);
-        else if (p.riemann == 1) RECONS(ASTRO_RMHD, 1);
-        else RECONS(ASTRO_RMHD, 0);
+cudaError_t launch_carried(const FaceArgs& a, bool given, cudaStream_t s) {
+    if (empty(a)) return cudaSuccess;
+    const int ri = a.p.riemann;
+    if (a.p.recon == ASTRO_RECON_PPM)
+        return ri == 2 ? OnePass<1, 2>::run(a, given, s)
+                       : (ri == 1 ? OnePass<1, 1>::run(a, given, s) : OnePass<1, 0>::run(a, given, s));
+    return ri == 2 ? OnePass<2, 2>::run(a, given, s)
+                   : (ri == 1 ? OnePass<2, 1>::run(a, given, s) : OnePass<2, 0>::run(a, given, s));
+}
+
+cudaError_t launch_all(const FaceArgs* dirs, void (*launched)(cudaStream_t), cudaStream_t s) {
+    FaceArgs3 a;
+    for (int d = 0; d < 3; ++d) {
+        a.d[d] = dirs[d];
+        // a third of the list each, the counters next to each other
+        const unsigned cap = dirs[d].fix_cap / 3;
+        a.d[d].fix_count = dirs[0].fix_count + d;
+        a.d[d].fix_list = dirs[0].fix_list + (size_t)d * cap;
+        a.d[d].fix_cap = cap;
     }
-#undef RECONS
-#undef FACE
-    if (me != cudaSuccess) return me;
-    return cudaGetLastError();
+    if (empty(a.d[0]) && empty(a.d[1]) && empty(a.d[2])) return cudaSuccess;
+    const AstroParams& p = a.d[0].p;
+    if (p.physics == ASTRO_SRHD)
+        return p.recon == 0 ? run_riemann<ASTRO_SRHD, 0>(a, launched, s)
+                            : (p.recon == 1 ? run_riemann<ASTRO_SRHD, 1>(a, launched, s)
+                                            : run_riemann<ASTRO_SRHD, 2>(a, launched, s));
+    return p.recon == 0 ? run_riemann<ASTRO_RMHD, 0>(a, launched, s)
+                        : (p.recon == 1 ? run_riemann<ASTRO_RMHD, 1>(a, launched, s)
+                                        : run_riemann<ASTRO_RMHD, 2>(a, launched, s));
 }
 
 }  // namespace astro_face32

@@ -870,9 +870,10 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
         mark(0, s);
         return cudaSuccess;
     }
+    FaceArgs dirs[3];
     for (int oi = 0; oi < 3; ++oi) {
         const int d = order[oi];
-        FaceArgs a;
+        FaceArgs& a = dirs[d];
         memset(&a, 0, sizeof(a));
         a.pr = pr; a.prf = prf; a.nx = g.nx; a.ny = g.ny; a.nz = g.nz; a.dir = d; a.b = b; a.p = p;
         a.ndiss = dissipation_fluxes(p, g);
@@ -886,20 +887,25 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
         a.fix_list = (unsigned*)(work + L.fix + 256);
         a.fix_cap = (unsigned)fix_capacity(g);
         a.speeds_out = (carried && d == 2) ? (void*)(work + L.Sz) : nullptr;
-        cudaError_t e = astro_face32::launch(a, false, s);
+        if (!carried) continue;
+        cudaError_t e = astro_face32::launch_carried(a, false, s);
         if (e != cudaSuccess) return e;
         mark(0, s);
-        if (carried && d == 0) {
+        if (d == 0) {
             FaceArgs c = a;
             c.ext[0] = b.hi[0] - b.lo;  // x-low faces of the updated cells
             c.F = work + L.FxC;
             c.aux = nullptr;
             c.speeds_out = nullptr;
             c.carried = work + L.Sz;
-            e = astro_face32::launch(c, true, s);
+            e = astro_face32::launch_carried(c, true, s);
             if (e != cudaSuccess) return e;
             mark(0, s);
         }
+    }
+    if (!carried) {
+        const cudaError_t e = astro_face32::launch_all(dirs, [](cudaStream_t t) { mark(0, t); }, s);
+        if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
