@@ -29,6 +29,7 @@
 #include "face64.cuh"
 
 #include <stdint.h>
+#include <string.h>
 
 using namespace astro;
 
@@ -263,6 +264,56 @@ __global__ void __launch_bounds__(T, PHYS == ASTRO_SRHD ? 8 : (RIEMANN == ASTRO_
     }
 }
 
+// One thread per face of one direction by the general evaluation, for steps that
+// depend on its last bit (Args::exact).  Faces of a 128^3 WENO5 hlld step 6.9 ms
+// against 1.9 ms above; a launch bound, a quotient of another form or both x fluxes
+// in one kernel change how the compiler fuses multiplications and additions, and
+// with it last bits.
+template <int RECON, int RIEMANN, bool GIVEN, int DIR>
+__global__ void __launch_bounds__(128) k_face_general(FaceArgs a) {
+    // grid: x over the (j, k) plane of the face block, y over its x layers;
+    // one 32-bit split of the in-plane index per thread
+    const unsigned e2 = (unsigned)a.ext[2];
+    const unsigned plane = (unsigned)a.ext[1] * e2;
+    const unsigned tp = blockIdx.x * blockDim.x + threadIdx.x;
+    if (tp >= plane) return;
+    const int c = (int)(tp % e2), bb = (int)(tp / e2);
+    for (int aa = blockIdx.y; aa < a.ext[0]; aa += gridDim.y) {
+        const int i = a.org[0] + aa, j = a.org[1] + bb, k = a.org[2] + c;
+        face_at<ASTRO_RMHD, RECON, RIEMANN, double, double, GIVEN, DIR>(a, i, j, k);
+    }
+}
+
+// z (with the speeds the carried x faces read), x, carried x, y: of those, the ones
+// this launch has buffers for
+template <int RECON, int RIEMANN>
+cudaError_t general_passes(const Args& a, cudaStream_t s) {
+    for (int pass = 0; pass < 4; ++pass) {
+        const int d = pass == 0 ? 2 : (pass == 3 ? 1 : 0);
+        const bool given = pass == 2;
+        if (given ? !a.FxC : !a.F[d]) continue;
+        FaceArgs f;
+        memset(&f, 0, sizeof(f));
+        f.pr = a.pr; f.nx = a.nx; f.ny = a.ny; f.nz = a.nz; f.dir = d; f.b = a.b; f.p = a.p;
+        for (int e = 0; e < 3; ++e) {
+            f.org[e] = a.b.lo;
+            f.ext[e] = a.b.hi[e] - a.b.lo + (e == d && !given ? 1 : 0);
+        }
+        f.F = given ? a.FxC : a.F[d];
+        f.aux = given ? nullptr : a.aux[d];
+        f.speeds_out = d == 2 ? a.speeds_out : nullptr;
+        f.carried = a.carried;
+        f.ndiss = a.ndiss;
+        const unsigned plane = (unsigned)f.ext[1] * (unsigned)f.ext[2];
+        const dim3 grd((plane + 127) / 128, (unsigned)(f.ext[0] < 65535 ? f.ext[0] : 65535));
+        if (given) k_face_general<RECON, RIEMANN, true, 0><<<grd, 128, 0, s>>>(f);
+        else if (d == 0) k_face_general<RECON, RIEMANN, false, 0><<<grd, 128, 0, s>>>(f);
+        else if (d == 1) k_face_general<RECON, RIEMANN, false, 1><<<grd, 128, 0, s>>>(f);
+        else k_face_general<RECON, RIEMANN, false, 2><<<grd, 128, 0, s>>>(f);
+    }
+    return cudaGetLastError();
+}
+
 template <int PH, int RE>
 void launch_riemann(const Args& a, unsigned blocks, cudaStream_t s) {
     if (a.p.riemann == 0) k_face64<PH, RE, 0><<<blocks, T, 0, s>>>(a);
@@ -275,6 +326,11 @@ void launch_riemann(const Args& a, unsigned blocks, cudaStream_t s) {
 cudaError_t launch(Args a, int sms, cudaStream_t s) {
     const long e[3] = {a.b.hi[0] - a.b.lo, a.b.hi[1] - a.b.lo, a.b.hi[2] - a.b.lo};
     if (e[0] <= 0 || e[1] <= 0 || e[2] <= 0) return cudaSuccess;
+    if (a.exact) {
+        const bool full = a.p.riemann == ASTRO_RIEMANN_HLLD_FULL;
+        if (a.p.recon == ASTRO_RECON_PPM) return full ? general_passes<1, 2>(a, s) : general_passes<1, 1>(a, s);
+        return full ? general_passes<2, 2>(a, s) : general_passes<2, 1>(a, s);
+    }
     long blocks[3] = {0, 0, 0};
     if (a.F[2]) blocks[2] = (e[0] * e[1] * ((e[2] + 1 + 30) / 31) + T / 32 - 1) / (T / 32);
     const long resident =

@@ -233,6 +233,7 @@ struct UpdArgs {
     double idd[3], idd2[3];
     int stage, nstages, rhs_only;
     int defer_c2p;       // learned con2prim: write U every stage, primitives later
+    int exact;           // flux differences divided to the last bit
     int frame_only;      // only the cells outside the updated range (the fused
                          // stage kernel updates the others)
     AstroParams p;
@@ -339,13 +340,48 @@ __global__ void __launch_bounds__(kUpdateBlock, PASSIVE ? 1 : 8) k_update(UpdArg
             // the update's instructions (float64 RMHD, 78^3 cells: 72 us with
             // them, 44 us without)
             const double i0 = a.idd[0], i1 = a.idd[1], i2 = a.idd[2];
+            bool divide = false;
+            if constexpr (sizeof(RF) == 8 && C2P != kC2PFast) {
+                if (a.exact) {
+                    // the quotients to the last bit: the product with the
+                    // rounded reciprocal corrected by its exact residual
+                    // (Markstein), as divisions where one is not finite
+                    auto quo = [](double x, double dd, double i) {
+                        const double q = x * i;
+                        return fma(fma(-dd, q, x), i, q);
+                    };
+                    bool ok = true;
 #pragma unroll
-            for (int v = 0; v < NM; ++v) {
-                double r = 0.0;
-                r -= (flux(0, v, 1) - flux(0, v, 0)) * i0;
-                r -= (flux(1, v, 1) - flux(1, v, 0)) * i1;
-                r -= (flux(2, v, 1) - flux(2, v, 0)) * i2;
-                rhs[v] = r;
+                    for (int v = 0; v < NM; ++v) {
+                        double r = 0.0;
+                        r -= quo(flux(0, v, 1) - flux(0, v, 0), a.dd[0], i0);
+                        r -= quo(flux(1, v, 1) - flux(1, v, 0), a.dd[1], i1);
+                        r -= quo(flux(2, v, 1) - flux(2, v, 0), a.dd[2], i2);
+                        rhs[v] = r;
+                        ok &= isfinite(r);
+                    }
+                    if (!ok) {
+#pragma unroll
+                        for (int v = 0; v < NM; ++v) {
+                            double r = 0.0;
+                            r -= (flux(0, v, 1) - flux(0, v, 0)) / a.dd[0];
+                            r -= (flux(1, v, 1) - flux(1, v, 0)) / a.dd[1];
+                            r -= (flux(2, v, 1) - flux(2, v, 0)) / a.dd[2];
+                            rhs[v] = r;
+                        }
+                    }
+                    divide = true;
+                }
+            }
+            if (!divide) {
+#pragma unroll
+                for (int v = 0; v < NM; ++v) {
+                    double r = 0.0;
+                    r -= (flux(0, v, 1) - flux(0, v, 0)) * i0;
+                    r -= (flux(1, v, 1) - flux(1, v, 0)) * i1;
+                    r -= (flux(2, v, 1) - flux(2, v, 0)) * i2;
+                    rhs[v] = r;
+                }
             }
             if (PHYS == ASTRO_RMHD) {
                 const double* q = a.prk;
@@ -798,6 +834,16 @@ void launch_update_t(const UpdArgs& a, dim3 grd, cudaStream_t s) {
     }
 }
 
+// Steps that keep the general evaluation's last bit in every part (faces, update,
+// con2prim): float64 "hlld" and "hlld_full" with the carried x-face speeds.  A contact
+// speed beside speeds that are not its face's divides by s - sM with no lower
+// bound, so a last bit anywhere in a stage comes out of the next one up to 1e9 times
+// larger (128^3 jets of W = 7: steps whose faces differed in last bits alone were up
+// to 1e-5 apart, 4 of 14 by more than 4e-8).  "hlle" has no such quotient, and with its own speeds s - sM is a wave's.
+inline bool exact_steps(const AstroParams& p) {
+    return p.precision == ASTRO_PREC_FP64 && carried_mode(p) && p.riemann != ASTRO_RIEMANN_HLLE;
+}
+
 // r_c2p's operation order (see r_f_eval): regrouped where nothing after it turns
 // its rounding into a jump, as PPM's flattening test does, and the float32 copy of
 // the mixed path (a last-bit change of a float32 velocity at W = 10 is 1e-5 of W^2)
@@ -813,7 +859,7 @@ cudaError_t launch_update(const UpdArgs& a, cudaStream_t s) {
         if (a.defer_c2p) launch_update_t<ASTRO_SRHD, kC2PDefer>(a, grd, s);
         else launch_update_t<ASTRO_SRHD, kC2PFast>(a, grd, s);
     } else if (a.defer_c2p) launch_update_t<ASTRO_RMHD, kC2PDefer>(a, grd, s);
-    else if (c2p_fast(a.p)) launch_update_t<ASTRO_RMHD, kC2PFast>(a, grd, s);
+    else if (a.rhs_only || (c2p_fast(a.p) && !exact_steps(a.p))) launch_update_t<ASTRO_RMHD, kC2PFast>(a, grd, s);
     else launch_update_t<ASTRO_RMHD, kC2PReference>(a, grd, s);
     mark(1, s);
     return cudaGetLastError();
@@ -834,7 +880,7 @@ int dissipation_fluxes(const AstroParams& p, const AstroGrid& g) {
 
 cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& b,
                         const double* pr, char* work, const Layout& L, cudaStream_t s,
-                        bool prf_ready = false) {
+                        bool prf_ready = false, bool exact = false) {
     const bool carried = carried_mode(p);
     const bool mixed = p.precision == ASTRO_PREC_MIXED;
     const int order[3] = {2, 0, 1};
@@ -851,6 +897,7 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
         memset(&a, 0, sizeof(a));
         a.pr = pr; a.nx = g.nx; a.ny = g.ny; a.nz = g.nz; a.b = b; a.p = p;
         a.ndiss = dissipation_fluxes(p, g);
+        a.exact = exact;
         for (int d = 0; d < 3; ++d) {
             if (d > 0 || !carried) a.F[d] = (double*)(work + L.F[d]);
             a.aux[d] = passive_fluxes(p) ? (double*)(work + L.aux[d]) : nullptr;
@@ -1758,13 +1805,14 @@ static int run_stage(const AstroParams* p, const AstroGrid* g, const Layout& L, 
                                dstf != nullptr, stats, s);
     const bool learned = p->c2p_guess == ASTRO_GUESS_LEARNED;
     const Bounds b = bounds_of(*p, *g);
-    cudaError_t e = face_passes(*p, *g, b, cur, w, L, s, prf_ready);
+    cudaError_t e = face_passes(*p, *g, b, cur, w, L, s, prf_ready, exact_steps(*p));
     if (e != cudaSuccess) return ASTRO_E_CUDA;
     UpdArgs u = update_args(*p, *g, b, w, L);
     u.pr0 = pr_in; u.prk = cur; u.U = (double*)(w + L.U); u.dst = dst;
     u.dstf = learned ? nullptr : dstf;
     u.dt = dt; u.stage = st; u.nstages = nst; u.rhs_only = 0; u.stats = stats;
     u.defer_c2p = learned ? 1 : 0;
+    u.exact = exact_steps(*p) ? 1 : 0;
     e = launch_update(u, s);
     if (e != cudaSuccess) return ASTRO_E_CUDA;
     if (learned) {
