@@ -798,7 +798,9 @@ cudaError_t launch_c2p_learned(const C2PArgs& a, cudaStream_t s) {
 
 // float32 copy of the first nm primitive rows (stage inputs that no
 // con2prim kernel of this library produced): four values per thread and turn where
-// the input is 16-byte aligned (262^3 cells, 9 variables: 370 -> 289 us)
+// both arrays are 16-byte aligned (262^3 cells, 9 variables: 370 -> 289 us).  The
+// copy is as aligned as the caller's workspace, which need only be a device buffer
+// that float64 values can lie in.
 __global__ void __launch_bounds__(256) k_prim_f32(const double* __restrict__ pr, float* __restrict__ prf,
                                                   size_t n, bool aligned) {
     const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
@@ -887,7 +889,8 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
     float* prf = mixed ? (float*)(work + L.prf) : nullptr;
     if (mixed && !prf_ready) {
         const size_t n = (size_t)(p.physics == ASTRO_SRHD ? 5 : 9) * g.nx * g.ny * g.nz;
-        k_prim_f32<<<sm_count_cached() * 8, 256, 0, s>>>(pr, prf, n, ((uintptr_t)pr & 15) == 0);
+        const bool aligned = (((uintptr_t)pr | (uintptr_t)prf) & 15) == 0;
+        k_prim_f32<<<sm_count_cached() * 8, 256, 0, s>>>(pr, prf, n, aligned);
         mark(2, s);
     }
     if (!mixed) {
