@@ -170,14 +170,18 @@ cudaError_t run_riemann(const FaceArgs3& a, void (*launched)(cudaStream_t), cuda
 
 }  // namespace
 
-cudaError_t launch_carried(const FaceArgs& a, bool given, cudaStream_t s) {
+cudaError_t launch_carried(const FaceArgs& a, bool given, void (*launched)(cudaStream_t), cudaStream_t s) {
     if (empty(a)) return cudaSuccess;
     const int ri = a.p.riemann;
+    cudaError_t e;
     if (a.p.recon == ASTRO_RECON_PPM)
-        return ri == 2 ? OnePass<1, 2>::run(a, given, s)
-                       : (ri == 1 ? OnePass<1, 1>::run(a, given, s) : OnePass<1, 0>::run(a, given, s));
-    return ri == 2 ? OnePass<2, 2>::run(a, given, s)
-                   : (ri == 1 ? OnePass<2, 1>::run(a, given, s) : OnePass<2, 0>::run(a, given, s));
+        e = ri == 2 ? OnePass<1, 2>::run(a, given, s)
+                    : (ri == 1 ? OnePass<1, 1>::run(a, given, s) : OnePass<1, 0>::run(a, given, s));
+    else
+        e = ri == 2 ? OnePass<2, 2>::run(a, given, s)
+                    : (ri == 1 ? OnePass<2, 1>::run(a, given, s) : OnePass<2, 0>::run(a, given, s));
+    if (e == cudaSuccess) launched(s);
+    return e;
 }
 
 cudaError_t launch_all(const FaceArgs* dirs, void (*launched)(cudaStream_t), cudaStream_t s) {

@@ -11,6 +11,7 @@ cudaError_t launch_all(const astro::FaceArgs* dirs, void (*launched)(cudaStream_
 // one direction's faces (a.dir), then its listed ones, for RMHD PPM and WENO5 in
 // the reference's flux mode, whose passes wait on one another; given: the x faces
 // with the carried z-face speeds
-cudaError_t launch_carried(const astro::FaceArgs& a, bool given, cudaStream_t s);
+cudaError_t launch_carried(const astro::FaceArgs& a, bool given, void (*launched)(cudaStream_t),
+                           cudaStream_t s);
 
 }  // namespace astro_face32

@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(128) k_face_general(FaceArgs a) {
 // z (with the speeds the carried x faces read), x, carried x, y: of those, the ones
 // this launch has buffers for
 template <int RECON, int RIEMANN>
-cudaError_t general_passes(const Args& a, cudaStream_t s) {
+cudaError_t general_passes(const Args& a, void (*launched)(cudaStream_t), cudaStream_t s) {
     for (int pass = 0; pass < 4; ++pass) {
         const int d = pass == 0 ? 2 : (pass == 3 ? 1 : 0);
         const bool given = pass == 2;
@@ -310,6 +310,7 @@ cudaError_t general_passes(const Args& a, cudaStream_t s) {
         else if (d == 0) k_face_general<RECON, RIEMANN, false, 0><<<grd, 128, 0, s>>>(f);
         else if (d == 1) k_face_general<RECON, RIEMANN, false, 1><<<grd, 128, 0, s>>>(f);
         else k_face_general<RECON, RIEMANN, false, 2><<<grd, 128, 0, s>>>(f);
+        launched(s);
     }
     return cudaGetLastError();
 }
@@ -323,13 +324,14 @@ void launch_riemann(const Args& a, unsigned blocks, cudaStream_t s) {
 
 }  // namespace
 
-cudaError_t launch(Args a, int sms, cudaStream_t s) {
+cudaError_t launch(Args a, int sms, void (*launched)(cudaStream_t), cudaStream_t s) {
     const long e[3] = {a.b.hi[0] - a.b.lo, a.b.hi[1] - a.b.lo, a.b.hi[2] - a.b.lo};
     if (e[0] <= 0 || e[1] <= 0 || e[2] <= 0) return cudaSuccess;
     if (a.exact) {
         const bool full = a.p.riemann == ASTRO_RIEMANN_HLLD_FULL;
-        if (a.p.recon == ASTRO_RECON_PPM) return full ? general_passes<1, 2>(a, s) : general_passes<1, 1>(a, s);
-        return full ? general_passes<2, 2>(a, s) : general_passes<2, 1>(a, s);
+        if (a.p.recon == ASTRO_RECON_PPM)
+            return full ? general_passes<1, 2>(a, launched, s) : general_passes<1, 1>(a, launched, s);
+        return full ? general_passes<2, 2>(a, launched, s) : general_passes<2, 1>(a, launched, s);
     }
     long blocks[3] = {0, 0, 0};
     if (a.F[2]) blocks[2] = (e[0] * e[1] * ((e[2] + 1 + 30) / 31) + T / 32 - 1) / (T / 32);
@@ -381,6 +383,7 @@ cudaError_t launch(Args a, int sms, cudaStream_t s) {
         else if (a.p.recon == 1) launch_riemann<ASTRO_RMHD, 1>(a, n, s);
         else launch_riemann<ASTRO_RMHD, 2>(a, n, s);
     }
+    launched(s);
     return cudaGetLastError();
 }
 

@@ -23,6 +23,7 @@ struct Args {
     int blocks_x, blocks_y, seg[2];
 };
 
-cudaError_t launch(Args a, int sms, cudaStream_t s);
+// launched: called after each kernel (the launch count and the kernel timing's events)
+cudaError_t launch(Args a, int sms, void (*launched)(cudaStream_t), cudaStream_t s);
 
 }  // namespace astro_face64

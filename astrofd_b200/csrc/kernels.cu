@@ -887,6 +887,7 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
     const bool mixed = p.precision == ASTRO_PREC_MIXED;
     const int order[3] = {2, 0, 1};
     float* prf = mixed ? (float*)(work + L.prf) : nullptr;
+    const auto launched = [](cudaStream_t t) { mark(0, t); };
     if (mixed && !prf_ready) {
         const size_t n = (size_t)(p.physics == ASTRO_SRHD ? 5 : 9) * g.nx * g.ny * g.nz;
         const bool aligned = (((uintptr_t)pr | (uintptr_t)prf) & 15) == 0;
@@ -906,19 +907,14 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
             a.aux[d] = passive_fluxes(p) ? (double*)(work + L.aux[d]) : nullptr;
         }
         if (carried) a.speeds_out = (double*)(work + L.Sz);
-        cudaError_t e = astro_face64::launch(a, sm_count_cached(), s);
-        if (e != cudaSuccess) return e;
-        mark(0, s);
-        if (!carried) return cudaSuccess;
+        const cudaError_t e = astro_face64::launch(a, sm_count_cached(), launched, s);
+        if (e != cudaSuccess || !carried) return e;
         a.F[0] = (double*)(work + L.F[0]);
         a.F[1] = a.F[2] = nullptr;
         a.speeds_out = nullptr;
         a.FxC = (double*)(work + L.FxC);
         a.carried = (const double*)(work + L.Sz);
-        e = astro_face64::launch(a, sm_count_cached(), s);
-        if (e != cudaSuccess) return e;
-        mark(0, s);
-        return cudaSuccess;
+        return astro_face64::launch(a, sm_count_cached(), launched, s);
     }
     FaceArgs dirs[3];
     for (int oi = 0; oi < 3; ++oi) {
@@ -938,9 +934,8 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
         a.fix_cap = (unsigned)fix_capacity(g);
         a.speeds_out = (carried && d == 2) ? (void*)(work + L.Sz) : nullptr;
         if (!carried) continue;
-        cudaError_t e = astro_face32::launch_carried(a, false, s);
+        cudaError_t e = astro_face32::launch_carried(a, false, launched, s);
         if (e != cudaSuccess) return e;
-        mark(0, s);
         if (d == 0) {
             FaceArgs c = a;
             c.ext[0] = b.hi[0] - b.lo;  // x-low faces of the updated cells
@@ -948,13 +943,12 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
             c.aux = nullptr;
             c.speeds_out = nullptr;
             c.carried = work + L.Sz;
-            e = astro_face32::launch_carried(c, true, s);
+            e = astro_face32::launch_carried(c, true, launched, s);
             if (e != cudaSuccess) return e;
-            mark(0, s);
         }
     }
     if (!carried) {
-        const cudaError_t e = astro_face32::launch_all(dirs, [](cudaStream_t t) { mark(0, t); }, s);
+        const cudaError_t e = astro_face32::launch_all(dirs, launched, s);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
