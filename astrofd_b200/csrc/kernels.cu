@@ -836,12 +836,14 @@ void launch_update_t(const UpdArgs& a, dim3 grd, cudaStream_t s) {
     }
 }
 
-// Steps that keep the general evaluation's last bit in every part (faces, update,
-// con2prim): float64 "hlld" and "hlld_full" with the carried x-face speeds.  A contact
+// Steps (plain and fixed-metric) that keep the general evaluation's last bit in every
+// part (faces, update, con2prim): float64 "hlld" and "hlld_full" with the carried x-face speeds.  A contact
 // speed beside speeds that are not its face's divides by s - sM with no lower
 // bound, so a last bit anywhere in a stage comes out of the next one up to 1e9 times
 // larger (128^3 jets of W = 7: steps whose faces differed in last bits alone were up
-// to 1e-5 apart, 4 of 14 by more than 4e-8).  "hlle" has no such quotient, and with its own speeds s - sM is a wave's.
+// to 1e-5 apart, 4 of 14 by more than 4e-8; fixed-metric steps of 12 such jets up to
+// 2.5e-5, 5 by more; a 72^3 Kerr-Schild step takes 1.68 ms so, 0.71 with the others'
+// faces).  "hlle" has no such quotient, and with its own speeds s - sM is a wave's.
 inline bool exact_steps(const AstroParams& p) {
     return p.precision == ASTRO_PREC_FP64 && carried_mode(p) && p.riemann != ASTRO_RIEMANN_HLLE;
 }
@@ -2187,13 +2189,14 @@ int astro_step_gr(const AstroParams* p, const AstroGrid* g, const AstroGR* gr,
         // the update writes U only; the sources are added to U with the
         // stage's weight of dt * rhs, then con2prim gives the primitives
         const double* fin = gr_flux_input(*gr, *g, cur, w, L.total, s);
-        cudaError_t e = face_passes(*p, *g, b, fin, w, L, s);
+        cudaError_t e = face_passes(*p, *g, b, fin, w, L, s, false, exact_steps(*p));
         if (e != cudaSuccess) return ASTRO_E_CUDA;
         double* dst = (st == nst - 1) ? pr_out : bufs[st % 2];
         UpdArgs u = update_args(*p, *g, b, w, L);
         u.pr0 = pr_in; u.prk = cur; u.U = U; u.dst = dst; u.dstf = nullptr;
         u.dt = dt; u.stage = st; u.nstages = nst; u.rhs_only = 0; u.stats = stats;
         u.defer_c2p = 1;
+        u.exact = exact_steps(*p) ? 1 : 0;
         e = launch_update(u, s);
         if (e != cudaSuccess) return ASTRO_E_CUDA;
         if (gr->metric != ASTRO_GR_MINKOWSKI) {
@@ -2213,7 +2216,8 @@ int astro_step_gr(const AstroParams* p, const AstroGrid* g, const AstroGR* gr,
             c.fb_cap = (unsigned)c2p_fb_capacity(*g);
             e = launch_c2p_learned(c, s);
         } else {
-            launch_c2p(*p, c2p_fast(*p), U, dst, (long)nc, stats, grid_for(nc, 128), s);
+            launch_c2p(*p, c2p_fast(*p) && !exact_steps(*p), U, dst, (long)nc, stats,
+                       grid_for(nc, 128), s);
             mark(2, s);
             e = cudaGetLastError();
         }

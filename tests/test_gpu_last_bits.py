@@ -1,0 +1,48 @@
+"""Float64 blocks whose schemes amplify a last bit (a contact speed beside speeds
+that are not its face's, divided by their unbounded difference) keep the general
+face evaluation, the quotients of the flux differences and the reference's con2prim
+order on every path to them, not in the plain steps alone.  Their face kernels tell
+the two evaluations apart: one per direction and one for the carried x faces."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from astrofd_b200 import _lib
+from astrofd_b200.core import grmhd_core, rmhd_core
+from states import make_state
+
+pytestmark = pytest.mark.gpu
+
+N = (9, 8, 11)
+
+
+def _setup(recon, riemann, flux_mode="reference"):
+    rmhd_core.configure(dict(GAMMA=4.0 / 3.0, P_MAX=2.0, V_MAX=0.9999, N_PASSIVE=0, PASSIVE_OFFSET=9,
+                             RECON=recon, RIEMANN=riemann, LIMITER="mc", RESISTIVE_ENABLED=False,
+                             RESISTIVITY=0.0, C2P_GUESS="reference", STAGE_KERNEL="split",
+                             FLUX_MODE=flux_mode, PRECISION="fp64"))
+    return torch.from_numpy(make_state(5, N, 3, "rmhd", stripes=False)).cuda()
+
+
+def _launches(f):
+    L = _lib.load()
+    before = L.astro_launch_count()
+    out = f()
+    return out, L.astro_launch_count() - before
+
+
+@pytest.mark.parametrize("recon", ["weno", "ppm"])
+@pytest.mark.parametrize("riemann,flux_mode,faces", [("hlld", "reference", 4), ("hlle", "reference", 2),
+                                                     ("hlld", "conservative", 1)])
+def test_gr_steps(recon, riemann, flux_mode, faces):
+    pr = _setup(recon, riemann, flux_mode)
+    d = (0.1, 0.1, 0.1)
+    plain = rmhd_core.step_ssprk3(pr, *d, 1e-3)
+    grmhd_core.configure(dict(GR_METRIC="minkowski", GR_MASS=0.0, ORTHONORMAL_FLUX=True))
+    gr, n = _launches(lambda: grmhd_core.step_ssprk3(pr, *d, 1e-3, 0, 3))
+    assert n == 3 * (faces + 2)  # and the update and the con2prim of each stage
+    # the con2prim runs in another kernel: the same operations, compiled apart
+    scale = plain.abs().flatten(1).amax(1).clamp_min(1e-300)
+    assert float(((gr - plain).abs().flatten(1).amax(1) / scale).max()) < 1e-9
