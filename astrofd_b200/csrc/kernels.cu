@@ -836,15 +836,19 @@ void launch_update_t(const UpdArgs& a, dim3 grd, cudaStream_t s) {
     }
 }
 
-// Steps (plain and fixed-metric) that keep the general evaluation's last bit in every
-// part (faces, update, con2prim): float64 "hlld" and "hlld_full" with the carried x-face speeds.  A contact
-// speed beside speeds that are not its face's divides by s - sM with no lower
-// bound, so a last bit anywhere in a stage comes out of the next one up to 1e9 times
-// larger (128^3 jets of W = 7: steps whose faces differed in last bits alone were up
-// to 1e-5 apart, 4 of 14 by more than 4e-8; fixed-metric steps of 12 such jets up to
-// 2.5e-5, 5 by more; a 72^3 Kerr-Schild step takes 1.68 ms so, 0.71 with the others'
-// faces).  "hlle" has no such quotient, and with its own speeds s - sM is a wave's.
-inline bool exact_steps(const AstroParams& p) {
+// Schemes that keep the general evaluation's last bit in every part (faces, update,
+// con2prim), in steps, fixed-metric steps and right-hand sides: float64 "hlld" and
+// "hlld_full" with the carried x-face speeds.  A contact speed beside speeds that are
+// not its face's divides by s - sM with no lower bound, so a last bit anywhere in a
+// stage comes out of the next one up to 1e9 times larger.  Jets of W = 7 at 128^3, the
+// fast evaluation against the general one: steps up to 1e-5 apart, 4 of 14 by more
+// than 4e-8; fixed-metric steps up to 2.5e-5, 5 of 12 by more; SSPRK3 loops over the
+// right-hand side (a user's own integrator) the same, though one right-hand side
+// moves by 4e-13 of its largest value only.  The fast faces would take 1.9 of 6.9 ms
+// per 128^3 WENO5 step, a 72^3 Kerr-Schild step with them 0.71 of 1.68 ms, a PPM
+// right-hand side of 90 x 61 x 103 cells 181 of 345 us.  "hlle" has no such quotient,
+// and with its own speeds s - sM is a wave's.
+inline bool exact_bits(const AstroParams& p) {
     return p.precision == ASTRO_PREC_FP64 && carried_mode(p) && p.riemann != ASTRO_RIEMANN_HLLE;
 }
 
@@ -852,7 +856,7 @@ inline bool exact_steps(const AstroParams& p) {
 // its rounding into a jump, as PPM's flattening test does, and the float32 copy of
 // the mixed path (a last-bit change of a float32 velocity at W = 10 is 1e-5 of W^2)
 inline bool c2p_fast(const AstroParams& p) {
-    return p.recon != ASTRO_RECON_PPM && p.precision == ASTRO_PREC_FP64;
+    return p.recon != ASTRO_RECON_PPM && p.precision == ASTRO_PREC_FP64 && !exact_bits(p);
 }
 
 cudaError_t launch_update(const UpdArgs& a, cudaStream_t s) {
@@ -863,7 +867,7 @@ cudaError_t launch_update(const UpdArgs& a, cudaStream_t s) {
         if (a.defer_c2p) launch_update_t<ASTRO_SRHD, kC2PDefer>(a, grd, s);
         else launch_update_t<ASTRO_SRHD, kC2PFast>(a, grd, s);
     } else if (a.defer_c2p) launch_update_t<ASTRO_RMHD, kC2PDefer>(a, grd, s);
-    else if (a.rhs_only || (c2p_fast(a.p) && !exact_steps(a.p))) launch_update_t<ASTRO_RMHD, kC2PFast>(a, grd, s);
+    else if (a.rhs_only ? !a.exact : c2p_fast(a.p)) launch_update_t<ASTRO_RMHD, kC2PFast>(a, grd, s);
     else launch_update_t<ASTRO_RMHD, kC2PReference>(a, grd, s);
     mark(1, s);
     return cudaGetLastError();
@@ -884,7 +888,7 @@ int dissipation_fluxes(const AstroParams& p, const AstroGrid& g) {
 
 cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& b,
                         const double* pr, char* work, const Layout& L, cudaStream_t s,
-                        bool prf_ready = false, bool exact = false) {
+                        bool prf_ready = false) {
     const bool carried = carried_mode(p);
     const bool mixed = p.precision == ASTRO_PREC_MIXED;
     const int order[3] = {2, 0, 1};
@@ -903,7 +907,7 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
         memset(&a, 0, sizeof(a));
         a.pr = pr; a.nx = g.nx; a.ny = g.ny; a.nz = g.nz; a.b = b; a.p = p;
         a.ndiss = dissipation_fluxes(p, g);
-        a.exact = exact;
+        a.exact = exact_bits(p);
         for (int d = 0; d < 3; ++d) {
             if (d > 0 || !carried) a.F[d] = (double*)(work + L.F[d]);
             a.aux[d] = passive_fluxes(p) ? (double*)(work + L.aux[d]) : nullptr;
@@ -972,6 +976,7 @@ UpdArgs update_args(const AstroParams& p, const AstroGrid& g, const Bounds& b, c
         u.idd[d] = 1.0 / u.dd[d];
         u.idd2[d] = 1.0 / (u.dd[d] * u.dd[d] + 1e-12);
     }
+    u.exact = exact_bits(p) ? 1 : 0;
     u.p = p;
     return u;
 }
@@ -1804,14 +1809,13 @@ static int run_stage(const AstroParams* p, const AstroGrid* g, const Layout& L, 
                                dstf != nullptr, stats, s);
     const bool learned = p->c2p_guess == ASTRO_GUESS_LEARNED;
     const Bounds b = bounds_of(*p, *g);
-    cudaError_t e = face_passes(*p, *g, b, cur, w, L, s, prf_ready, exact_steps(*p));
+    cudaError_t e = face_passes(*p, *g, b, cur, w, L, s, prf_ready);
     if (e != cudaSuccess) return ASTRO_E_CUDA;
     UpdArgs u = update_args(*p, *g, b, w, L);
     u.pr0 = pr_in; u.prk = cur; u.U = (double*)(w + L.U); u.dst = dst;
     u.dstf = learned ? nullptr : dstf;
     u.dt = dt; u.stage = st; u.nstages = nst; u.rhs_only = 0; u.stats = stats;
     u.defer_c2p = learned ? 1 : 0;
-    u.exact = exact_steps(*p) ? 1 : 0;
     e = launch_update(u, s);
     if (e != cudaSuccess) return ASTRO_E_CUDA;
     if (learned) {
@@ -2189,14 +2193,13 @@ int astro_step_gr(const AstroParams* p, const AstroGrid* g, const AstroGR* gr,
         // the update writes U only; the sources are added to U with the
         // stage's weight of dt * rhs, then con2prim gives the primitives
         const double* fin = gr_flux_input(*gr, *g, cur, w, L.total, s);
-        cudaError_t e = face_passes(*p, *g, b, fin, w, L, s, false, exact_steps(*p));
+        cudaError_t e = face_passes(*p, *g, b, fin, w, L, s);
         if (e != cudaSuccess) return ASTRO_E_CUDA;
         double* dst = (st == nst - 1) ? pr_out : bufs[st % 2];
         UpdArgs u = update_args(*p, *g, b, w, L);
         u.pr0 = pr_in; u.prk = cur; u.U = U; u.dst = dst; u.dstf = nullptr;
         u.dt = dt; u.stage = st; u.nstages = nst; u.rhs_only = 0; u.stats = stats;
         u.defer_c2p = 1;
-        u.exact = exact_steps(*p) ? 1 : 0;
         e = launch_update(u, s);
         if (e != cudaSuccess) return ASTRO_E_CUDA;
         if (gr->metric != ASTRO_GR_MINKOWSKI) {
@@ -2216,8 +2219,7 @@ int astro_step_gr(const AstroParams* p, const AstroGrid* g, const AstroGR* gr,
             c.fb_cap = (unsigned)c2p_fb_capacity(*g);
             e = launch_c2p_learned(c, s);
         } else {
-            launch_c2p(*p, c2p_fast(*p) && !exact_steps(*p), U, dst, (long)nc, stats,
-                       grid_for(nc, 128), s);
+            launch_c2p(*p, c2p_fast(*p), U, dst, (long)nc, stats, grid_for(nc, 128), s);
             mark(2, s);
             e = cudaGetLastError();
         }

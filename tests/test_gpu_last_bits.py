@@ -5,7 +5,6 @@ order on every path to them, not in the plain steps alone.  Their face kernels t
 the two evaluations apart: one per direction and one for the carried x faces."""
 import ctypes as C
 
-import numpy as np
 import pytest
 import torch
 
@@ -46,3 +45,26 @@ def test_gr_steps(recon, riemann, flux_mode, faces):
     # the con2prim runs in another kernel: the same operations, compiled apart
     scale = plain.abs().flatten(1).amax(1).clamp_min(1e-300)
     assert float(((gr - plain).abs().flatten(1).amax(1) / scale).max()) < 1e-9
+
+
+@pytest.mark.parametrize("recon", ["weno", "ppm"])
+@pytest.mark.parametrize("riemann,flux_mode,faces", [("hlld", "reference", 4), ("hlle", "reference", 2),
+                                                     ("hlld", "conservative", 1)])
+@pytest.mark.parametrize("entry", ["rhs", "static", "gr"])
+def test_right_hand_sides(entry, recon, riemann, flux_mode, faces):
+    L = _lib.load()
+    pr = _setup(recon, riemann, flux_mode)
+    shape, d = tuple(pr.shape[1:]), (0.1, 0.1, 0.1)
+    plain, n = _launches(lambda: rmhd_core.engine().rhs(pr, *shape, *d))
+    if entry == "static":
+        out = torch.empty_like(pr)
+        g = _lib.AstroGrid(*pr.shape, *d)
+        rc, n = _launches(lambda: L.astro_rhs_static(
+            C.byref(rmhd_core.engine().p), C.byref(g), C.c_void_p(pr.data_ptr()),
+            C.c_void_p(out.data_ptr()), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        assert rc == 0 and torch.equal(out, plain)
+    elif entry == "gr":
+        grmhd_core.configure(dict(GR_METRIC="minkowski", GR_MASS=0.0, ORTHONORMAL_FLUX=True))
+        out, n = _launches(lambda: grmhd_core.compute_rhs_grmhd(pr, *d, 0, 3))
+        assert torch.equal(out, plain)
+    assert n == faces + 1  # and the update
