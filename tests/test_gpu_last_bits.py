@@ -5,11 +5,13 @@ order on every path to them, not in the plain steps alone.  Their face kernels t
 the two evaluations apart: one per direction and one for the carried x faces."""
 import ctypes as C
 
+import numpy as np
 import pytest
 import torch
 
 from astrofd_b200 import _lib
 from astrofd_b200.core import grmhd_core, rmhd_core
+from astrofd_b200.workloads import rmhd_jet
 from states import make_state
 
 pytestmark = pytest.mark.gpu
@@ -68,3 +70,34 @@ def test_right_hand_sides(entry, recon, riemann, flux_mode, faces):
         out, n = _launches(lambda: grmhd_core.compute_rhs_grmhd(pr, *d, 0, 3))
         assert torch.equal(out, plain)
     assert n == faces + 1  # and the update
+
+
+@pytest.mark.parametrize("riemann,flux_mode", [("hlle", "conservative"), ("hlld", "conservative"),
+                                               ("hlle", "reference")])
+@pytest.mark.parametrize("recon", ["ppm", "weno"])
+def test_a_loop_over_right_hand_sides_and_batches_is_the_step(recon, riemann, flux_mode):
+    """PPM's flattening compares neighbouring cells, whose pressures differ by the
+    conversion's rounding alone where they began equal: the batch conversion keeps
+    the order of operations that the configured step's has.  What remains is the
+    conversion's tolerance of 1e-10 max(1, tau)."""
+    ng, n = 3, 32
+    pr = _setup(recon, riemann, flux_mode)
+    pr = torch.from_numpy(np.ascontiguousarray(rmhd_jet(n, ng)[:9])).cuda()
+    e, shape, d = rmhd_core.engine(), tuple(pr.shape[1:]), (1.0 / n,) * 3
+    dt = 0.2 / n
+    step = rmhd_core.step_ssprk3(pr, *d, dt)
+
+    def rhs(q):
+        return e.rhs(q, *shape, *d).reshape(9, -1)
+
+    def prims(U):
+        return e.c2p_array(U).reshape(pr.shape)
+
+    U0 = e.p2c_array(pr)
+    U1 = U0 + dt * rhs(pr)
+    q = prims(U1)
+    U2 = 0.75 * U0 + 0.25 * (U1 + dt * rhs(q))
+    q = prims(U2)
+    loop = prims(U0 / 3.0 + 2.0 / 3.0 * (U2 + dt * rhs(q)))
+    scale = step.abs().flatten(1).amax(1).clamp_min(1e-300)
+    assert float(((loop - step).abs().flatten(1).amax(1) / scale).max()) < 1e-8
