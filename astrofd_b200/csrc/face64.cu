@@ -237,9 +237,9 @@ __device__ __forceinline__ void walk(const Args& a, double* sh, unsigned block) 
 
 // Blocks per SM: SRHD 8 (64 registers: 4 blocks at 128 take 723 against 683 us for
 // a 128^3 PPM step's faces, 113 against 89 us for a 64^3 MUSCL one's); RMHD 4 (128
-// registers); "hlld_full" 2.
+// registers).
 template <int PHYS, int RECON, int RIEMANN>
-__global__ void __launch_bounds__(T, PHYS == ASTRO_SRHD ? 8 : (RIEMANN == ASTRO_RIEMANN_HLLD_FULL ? 2 : 4))
+__global__ void __launch_bounds__(T, PHYS == ASTRO_SRHD ? 8 : 4)
     k_face64(const __grid_constant__ Args a) {
     constexpr int NM = PHYS == ASTRO_SRHD ? 5 : 9;
     __shared__ double sh[NM * T];
@@ -306,8 +306,10 @@ cudaError_t general_passes(const Args& a, void (*launched)(cudaStream_t), cudaSt
         f.ndiss = a.ndiss;
         const unsigned plane = (unsigned)f.ext[1] * (unsigned)f.ext[2];
         const dim3 grd((plane + 127) / 128, (unsigned)(f.ext[0] < 65535 ? f.ext[0] : 65535));
-        if (given) k_face_general<RECON, RIEMANN, true, 0><<<grd, 128, 0, s>>>(f);
-        else if (d == 0) k_face_general<RECON, RIEMANN, false, 0><<<grd, 128, 0, s>>>(f);
+        if (given) {
+            if constexpr (RECON != ASTRO_RECON_MUSCL)
+                k_face_general<RECON, RIEMANN, true, 0><<<grd, 128, 0, s>>>(f);
+        } else if (d == 0) k_face_general<RECON, RIEMANN, false, 0><<<grd, 128, 0, s>>>(f);
         else if (d == 1) k_face_general<RECON, RIEMANN, false, 1><<<grd, 128, 0, s>>>(f);
         else k_face_general<RECON, RIEMANN, false, 2><<<grd, 128, 0, s>>>(f);
         launched(s);
@@ -317,9 +319,9 @@ cudaError_t general_passes(const Args& a, void (*launched)(cudaStream_t), cudaSt
 
 template <int PH, int RE>
 void launch_riemann(const Args& a, unsigned blocks, cudaStream_t s) {
+    // "hlld_full" is always Args::exact
     if (a.p.riemann == 0) k_face64<PH, RE, 0><<<blocks, T, 0, s>>>(a);
-    else if (a.p.riemann == 1) k_face64<PH, RE, 1><<<blocks, T, 0, s>>>(a);
-    else if constexpr (PH == ASTRO_RMHD) k_face64<PH, RE, 2><<<blocks, T, 0, s>>>(a);
+    else k_face64<PH, RE, 1><<<blocks, T, 0, s>>>(a);
 }
 
 }  // namespace
@@ -329,14 +331,14 @@ cudaError_t launch(Args a, int sms, void (*launched)(cudaStream_t), cudaStream_t
     if (e[0] <= 0 || e[1] <= 0 || e[2] <= 0) return cudaSuccess;
     if (a.exact) {
         const bool full = a.p.riemann == ASTRO_RIEMANN_HLLD_FULL;
+        if (a.p.recon == ASTRO_RECON_MUSCL) return general_passes<0, 2>(a, launched, s);
         if (a.p.recon == ASTRO_RECON_PPM)
             return full ? general_passes<1, 2>(a, launched, s) : general_passes<1, 1>(a, launched, s);
         return full ? general_passes<2, 2>(a, launched, s) : general_passes<2, 1>(a, launched, s);
     }
     long blocks[3] = {0, 0, 0};
     if (a.F[2]) blocks[2] = (e[0] * e[1] * ((e[2] + 1 + 30) / 31) + T / 32 - 1) / (T / 32);
-    const long resident =
-        (long)sms * (a.p.physics == ASTRO_SRHD ? 8 : (a.p.riemann == ASTRO_RIEMANN_HLLD_FULL ? 2 : 4));
+    const long resident = (long)sms * (a.p.physics == ASTRO_SRHD ? 8 : 4);
     for (int d = 0; d < 2; ++d) {
         if (!a.F[d]) continue;
         // A longer walk repeats fewer reconstructions at its start (about 0.6 of a

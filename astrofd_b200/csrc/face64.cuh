@@ -16,8 +16,8 @@ struct Args {
     double* FxC;         // x faces: also the fluxes with the carried speeds, or null
     const double* carried;  // those speeds (an earlier launch's speeds_out)
     int ndiss;
-    bool exact;          // the general evaluation, to its last bit (RMHD PPM and WENO5
-                         // with "hlld" or "hlld_full")
+    bool exact;          // the general evaluation, to its last bit (RMHD "hlld_full", and
+                         // PPM and WENO5 with "hlld")
     AstroParams p;
     // set by launch(): thread blocks of x, y (z follow) and faces per thread
     int blocks_x, blocks_y, seg[2];

@@ -837,19 +837,22 @@ void launch_update_t(const UpdArgs& a, dim3 grd, cudaStream_t s) {
 }
 
 // Schemes that keep the general evaluation's last bit in every part (faces, update,
-// con2prim), in steps, fixed-metric steps and right-hand sides: float64 "hlld" and
-// "hlld_full" with the carried x-face speeds.  A contact speed beside speeds that are
-// not its face's divides by s - sM with no lower bound, so a last bit anywhere in a
+// con2prim), in steps, fixed-metric steps and right-hand sides: float64 "hlld" with the
+// carried x-face speeds, and "hlld_full".  A contact speed beside speeds that are not
+// its face's divides by s - sM with no lower bound, so a last bit anywhere in a
 // stage comes out of the next one up to 1e9 times larger.  Jets of W = 7 at 128^3, the
 // fast evaluation against the general one: steps up to 1e-5 apart, 4 of 14 by more
 // than 4e-8; fixed-metric steps up to 2.5e-5, 5 of 12 by more; SSPRK3 loops over the
 // right-hand side (a user's own integrator) the same, though one right-hand side
 // moves by 4e-13 of its largest value only.  The fast faces would take 1.9 of 6.9 ms
 // per 128^3 WENO5 step, a 72^3 Kerr-Schild step with them 0.71 of 1.68 ms, a PPM
-// right-hand side of 90 x 61 x 103 cells 181 of 345 us.  "hlle" has no such quotient,
-// and with its own speeds s - sM is a wave's.
+// right-hand side of 90 x 61 x 103 cells 181 of 345 us.  "hlld_full" divides by
+// D (s - v) - Bn^2, which has no bound with any speeds: steps of 40^3 jets 0.2 to 2 of
+// their largest value apart.  "hlle" has no such quotient, and with its own speeds
+// s - sM is a wave's.
 inline bool exact_bits(const AstroParams& p) {
-    return p.precision == ASTRO_PREC_FP64 && carried_mode(p) && p.riemann != ASTRO_RIEMANN_HLLE;
+    if (p.physics != ASTRO_RMHD || p.precision != ASTRO_PREC_FP64) return false;
+    return p.riemann == ASTRO_RIEMANN_HLLD_FULL || (carried_mode(p) && p.riemann == ASTRO_RIEMANN_HLLD);
 }
 
 // r_c2p's operation order (see r_f_eval): regrouped where nothing after it turns

@@ -101,3 +101,16 @@ def test_a_loop_over_right_hand_sides_and_batches_is_the_step(recon, riemann, fl
     loop = prims(U0 / 3.0 + 2.0 / 3.0 * (U2 + dt * rhs(q)))
     scale = step.abs().flatten(1).amax(1).clamp_min(1e-300)
     assert float(((loop - step).abs().flatten(1).amax(1) / scale).max()) < 1e-8
+
+
+@pytest.mark.parametrize("recon,flux_mode,faces", [("muscl", "reference", 3), ("muscl", "conservative", 3),
+                                                   ("ppm", "conservative", 3), ("weno", "conservative", 3),
+                                                   ("weno", "reference", 4)])
+def test_hlld_full_with_any_speeds(recon, flux_mode, faces):
+    """"hlld_full" also divides by D (s - v) - Bn^2; so with its own speeds too."""
+    pr = _setup(recon, "hlld_full", flux_mode)
+    shape, d = tuple(pr.shape[1:]), (0.1, 0.1, 0.1)
+    _, n = _launches(lambda: rmhd_core.engine().rhs(pr, *shape, *d))
+    assert n == faces + 1
+    _, n = _launches(lambda: rmhd_core.step_ssprk2(pr, *d, 1e-3))
+    assert n == 2 * (faces + 1)
