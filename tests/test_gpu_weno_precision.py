@@ -1,0 +1,112 @@
+"""Rounding of the float64 WENO5 faces, against 80-bit arithmetic: a right-hand side
+is the difference of two nearly equal fluxes, so in a fast beam it shows every last
+bit of a face velocity, W^2 times larger."""
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.skipif(np.finfo(np.longdouble).eps > 1e-18, reason="long double is float64 here")
+
+CFG = dict(GAMMA=5.0 / 3.0, P_MAX=2.0, V_MAX=0.9999, N_PASSIVE=0, PASSIVE_OFFSET=5, RECON="weno",
+           LIMITER="mc", RIEMANN="hlle", FLUX_MODE="reference", PRECISION="fp64")
+N, D = (14, 24, 26), (1.0 / 14, 1.0 / 24, 1.0 / 26)
+
+
+def _beam(seed):
+    """A W ~ 7 beam with a steep head and shear layer: one smooth stencil has nearly
+    all of the weight there, where the last bits of the weights show."""
+    r = np.random.default_rng(seed)
+    S = tuple(n + 6 for n in N)
+    x, y, z = np.meshgrid(*[(np.arange(s) - 2.5) / (s - 6) for s in S], indexing="ij")
+    s = 0.25 * (1.0 - np.tanh((np.hypot(y - 0.5, z - 0.5) - 0.2) / 0.03)) * (1.0 - np.tanh((x - 0.6) / 0.03))
+    pr = np.zeros((5,) + S)
+    pr[0] = 1.0 - 0.9 * s
+    pr[1] = 0.989 * s
+    pr[2] = 0.04 * s * np.sin(9.0 * x + 3.0 * z) + r.uniform(-0.002, 0.002, S)
+    pr[3] = 0.04 * s * np.cos(8.0 * x + 2.0 * y) + r.uniform(-0.002, 0.002, S)
+    pr[4] = 0.01 * (1.0 + 0.3 * s * np.sin(11.0 * x))
+    return pr
+
+
+def weno5(a, b, c, d, e):
+    T = a.dtype.type
+    k, eps = T(13.0 / 12.0), T(1e-12)
+    t = [a - 2 * b + c, b - 2 * c + d, c - 2 * d + e]
+    u = [a - 4 * b + 3 * c, b - d, 3 * c - 4 * d + e]
+    q = [T(1 / 3) * a - T(7 / 6) * b + T(11 / 6) * c, -T(1 / 6) * b + T(5 / 6) * c + T(1 / 3) * d,
+         T(1 / 3) * c + T(5 / 6) * d - T(1 / 6) * e]
+    w = [T(g) / (eps + k * (ti * ti) + T(0.25) * (ui * ui)) ** 2 for g, ti, ui in zip((0.1, 0.6, 0.3), t, u)]
+    s = w[0] + w[1] + w[2]
+    return sum((wi / s) * qi for wi, qi in zip(w, q))
+
+
+def rhs(pr, T, face_value=weno5):
+    """SRHD WENO5 HLLE (Gamma = 5/3, no floor active) in arithmetic T."""
+    pr = pr.astype(T)
+    G = T(5.0 / 3.0)
+
+    def states(q):
+        rho, v, p = q[0], q[1:4], q[4]
+        W = 1 / np.sqrt(1 - (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]))
+        w = rho * (1 + G / (G - 1) * p / rho)
+        U = np.stack([rho * W, w * W * W * v[0], w * W * W * v[1], w * W * W * v[2], w * W * W - p - rho * W])
+        return U, np.sqrt(G * p / w)
+
+    out = np.zeros_like(pr)
+    n = pr.shape[1:]
+    core = tuple(slice(3, m - 3) for m in n)
+    for d in range(3):
+        def at(o):  # cells lo + o .. of the faces lo .. hi
+            s = list(core)
+            s[d] = slice(3 + o, n[d] - 2 + o)
+            return pr[(slice(None),) + tuple(s)]
+        L = face_value(at(-3), at(-2), at(-1), at(0), at(1))
+        R = face_value(at(2), at(1), at(0), at(-1), at(-2))
+        (UL, cL), (UR, cR) = states(L), states(R)
+
+        def flux(q, U):
+            F = U * q[1 + d]
+            F[1 + d] += q[4]
+            F[4] += q[4] * q[1 + d]
+            return F
+        FL, FR = flux(L, UL), flux(R, UR)
+        lam = [(q[1 + d] + s * c) / (1 + s * q[1 + d] * c) for q, c in ((L, cL), (R, cR)) for s in (-1, 1)]
+        sL, sR = np.minimum(lam[0], lam[2]), np.maximum(lam[1], lam[3])
+        F = (sR * FL - sL * FR + sL * sR * (UR - UL)) / (sR - sL + T(1e-12))
+        F = np.where(sL >= 0, FL, np.where(sR <= 0, FR, F))
+        hi, lo = [slice(None)] * 4, [slice(None)] * 4
+        hi[1 + d], lo[1 + d] = slice(1, None), slice(None, -1)
+        out[(slice(None),) + core] -= (F[tuple(hi)] - F[tuple(lo)]) / T(D[d])
+    return out
+
+
+def _error(got, exact):
+    e = [np.sqrt(((g - x) ** 2).sum() / (x ** 2).sum()) for g, x in zip(got.astype(np.longdouble), exact)]
+    return np.array(e, float)
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_the_restatement_is_the_oracles_scheme(seed):
+    pr = _beam(seed)
+    exact = rhs(pr, np.longdouble)
+    ref = O.rhs(O.params_from_config("srhd", CFG), pr, *D)
+    assert np.all(_error(ref, exact) < 1e-11)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("seed", [1, 2, 3])
+def test_face_rounding(seed):
+    """The reference's own form, weights over their sum times polynomials, rounds each
+    face value by about one half ulp rms (1.0 measured); the differences from the middle
+    polynomial, weighted, by 0.5 to 0.6.  So the right-hand side's error is below the
+    oracle's; 0.8 of it allows for the rest of the face."""
+    import torch
+    from astrofd_b200.core import srhd_core
+    pr = _beam(seed)
+    exact = rhs(pr, np.longdouble)
+    srhd_core.configure(CFG)
+    got = srhd_core.compute_rhs_weno(torch.from_numpy(pr).cuda(), *pr.shape[1:], *D).cpu().numpy()
+    ref = O.rhs(O.params_from_config("srhd", CFG), pr, *D)
+    e, r = _error(got, exact), _error(ref, exact)
+    assert np.all(e <= 0.8 * r), (e, r)
