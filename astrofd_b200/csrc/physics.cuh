@@ -458,7 +458,7 @@ AHD void s_face(const Phys<R>& P, int n, R* qL, R* qR, R* F, R& sL, R& sR, int n
     R csL = s_sound_speed(P, qL[0], qL[4]), csR = s_sound_speed(P, qR[0], qR[4]);
     eig_speeds(qL[1 + n], csL, lmL, lpL);
     eig_speeds(qR[1 + n], csR, lmR, lpR);
-    sL = rmin(lmL, lmR);
+    sL = kRecip<R> && sizeof(R) == 8 ? rmin(lmR, lmL) : rmin(lmL, lmR);  // fd: see r_face_states
     sR = rmax(lpL, lpR);
     if (RIEMANN == ASTRO_RIEMANN_HLLC)
         hllc5(n, UL, UR, FL, FR, sL, sR, qL[4], qR[4], qL[1 + n], qR[1 + n], F);
@@ -753,7 +753,10 @@ AHD void r_face_states(const Phys<fd>& P, int n, fd* qL, fd* qR, fd* UL, fd* UR,
     r_flux_u(P, n, qR, UR, FR, BBR, vbR);
     eig_speeds(qL[1 + n], r_fast_speed_from(P, qL[4], rhL, b2L), lmL, lpL);
     eig_speeds(qR[1 + n], r_fast_speed_from(P, qR[4], rhR, b2R), lmR, lpR);
-    sL = rmin(lmL, lmR);
+    // a NaN of the left state stays in sL (rmin takes its second argument then) and one of
+    // the right state in sR: a state beyond the reciprocals' range sends the face to the
+    // general evaluation even where the other side's flux alone is taken
+    sL = rmin(lmR, lmL);
     sR = rmax(lpL, lpR);
 }
 
