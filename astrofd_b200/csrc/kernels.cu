@@ -343,20 +343,15 @@ __global__ void __launch_bounds__(kUpdateBlock, PASSIVE ? 1 : 8) k_update(UpdArg
             bool divide = false;
             if constexpr (sizeof(RF) == 8 && C2P != kC2PFast) {
                 if (a.exact) {
-                    // the quotients to the last bit: the product with the
-                    // rounded reciprocal corrected by its exact residual
-                    // (Markstein), as divisions where one is not finite
-                    auto quo = [](double x, double dd, double i) {
-                        const double q = x * i;
-                        return fma(fma(-dd, q, x), i, q);
-                    };
+                    // the quotients to the last bit, as divisions where one
+                    // is not finite
                     bool ok = true;
 #pragma unroll
                     for (int v = 0; v < NM; ++v) {
                         double r = 0.0;
-                        r -= quo(flux(0, v, 1) - flux(0, v, 0), a.dd[0], i0);
-                        r -= quo(flux(1, v, 1) - flux(1, v, 0), a.dd[1], i1);
-                        r -= quo(flux(2, v, 1) - flux(2, v, 0), a.dd[2], i2);
+                        r -= quot_(flux(0, v, 1) - flux(0, v, 0), a.dd[0], i0);
+                        r -= quot_(flux(1, v, 1) - flux(1, v, 0), a.dd[1], i1);
+                        r -= quot_(flux(2, v, 1) - flux(2, v, 0), a.dd[2], i2);
                         rhs[v] = r;
                         ok &= isfinite(r);
                     }
@@ -733,6 +728,14 @@ __global__ void k_c2p_features(const double* U, float* x, long count) {
 __global__ void k_rcp_f64(const double* x, double* y, long n) {
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
         y[i] = rcp_nr(x[i]);
+}
+
+// the float64 faces' reciprocals and roots and the update's quotients over an array
+// (test hook)
+__global__ void k_math_f64(int op, const double* x, double d, double inv, double* y, long n) {
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+        y[i] = op == 0 ? rcp_(fd(x[i])).v : (op == 1 ? rsq_(fd(x[i])).v : (op == 2 ? rsqrt_(fd(x[i])).v
+                                                                               : quot_(x[i], d, inv)));
 }
 
 int g_sm_count = 0;
@@ -1897,6 +1900,15 @@ int astro_debug_rcp_f64(const double* x, double* y, int64_t n, void* stream) {
     if (!x || !y) return ASTRO_E_INVALID;
     const int grid = (int)((n + 255) / 256 < 65535 ? (n + 255) / 256 : 65535);
     k_rcp_f64<<<grid, 256, 0, (cudaStream_t)stream>>>(x, y, (long)n);
+    return cudaGetLastError() == cudaSuccess ? ASTRO_OK : ASTRO_E_CUDA;
+}
+
+int astro_debug_math_f64(int op, const double* x, double d, double* y, int64_t n, void* stream) {
+    if (op < 0 || op > 3 || n < 0) return ASTRO_E_INVALID;
+    if (n == 0) return ASTRO_OK;
+    if (!x || !y) return ASTRO_E_INVALID;
+    const int grid = (int)((n + 255) / 256 < 65535 ? (n + 255) / 256 : 65535);
+    k_math_f64<<<grid, 256, 0, (cudaStream_t)stream>>>(op, x, d, 1.0 / d, y, (long)n);
     return cudaGetLastError() == cudaSuccess ? ASTRO_OK : ASTRO_E_CUDA;
 }
 
