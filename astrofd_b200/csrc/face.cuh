@@ -30,6 +30,8 @@ struct FaceArgs {
     unsigned* fix_count;
     unsigned* fix_list;
     unsigned fix_cap;
+    int fix_before;      // earlier passes whose faces stand before this one's in the
+                         // list; their counts are in front of fix_count
 };
 
 // One face: reconstruct, floor, p2c, flux, speeds, Riemann in arithmetic R,

@@ -8,6 +8,14 @@ using namespace astro;
 namespace astro_face32 {
 namespace {
 
+// first place of this pass in the list of faces to recompute: behind the faces that the
+// passes before it (complete by now: one stream) have counted
+__device__ __forceinline__ size_t fix_base(const FaceArgs& a) {
+    size_t n = 0;
+    for (int q = 1; q <= a.fix_before; ++q) n += a.fix_count[-q];
+    return n;
+}
+
 // float32 face pass of one direction (the float64 passes are face64.cu's)
 template <int PHYS, int RECON, int RIEMANN, bool GIVEN, int DIR>
 __global__ void __launch_bounds__(128) k_face(FaceArgs a) {
@@ -22,7 +30,7 @@ __global__ void __launch_bounds__(128) k_face(FaceArgs a) {
         const int i = a.org[0] + aa, j = a.org[1] + bb, k = a.org[2] + c;
         const bool ok = face_at<PHYS, RECON, RIEMANN, float, float, GIVEN, DIR>(a, i, j, k);
         if (!ok && a.fix_list) {
-            const unsigned slot = atomicAdd(a.fix_count, 1u);
+            const size_t slot = fix_base(a) + atomicAdd(a.fix_count, 1u);
             if (slot < a.fix_cap) a.fix_list[slot] = (unsigned)aa * plane + tp;
         }
     }
@@ -51,17 +59,18 @@ __device__ __forceinline__ bool face_stored_finite(const FaceArgs& a, size_t nc,
 // float64 recomputation of the faces a float32 pass listed as non-finite
 // (float32 overflows where float64 does not, e.g. squared WENO smoothness
 // indicators of a state whose fields have grown past ~1e9).  If more faces
-// failed than the list holds (the counter keeps counting past its capacity),
-// the list is incomplete: every face of the pass is then checked and the
+// failed than the list has room for (the counter keeps counting past it), the
+// pass's part of it is incomplete: every face of the pass is then checked and the
 // non-finite ones are recomputed, so no float32 failure is left in place.
 template <int PHYS, int RECON, int RIEMANN, bool GIVEN, int DIR>
 __device__ __forceinline__ void fix_pass(const FaceArgs& a) {
     constexpr int NM = PHYS == ASTRO_SRHD ? 5 : 9;
     const unsigned cnt = *a.fix_count;
-    if (cnt <= a.fix_cap) {
+    const size_t base = fix_base(a);
+    if (base + cnt <= a.fix_cap) {
         for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < cnt;
              q += gridDim.x * blockDim.x) {
-            const long t = a.fix_list[q];
+            const long t = a.fix_list[base + q];
             const int c = (int)(t % a.ext[2]);
             const long r = t / a.ext[2];
             const int bb = (int)(r % a.ext[1]);
@@ -144,8 +153,6 @@ struct OnePass {
 // (SSPRK3 step of a 75 x 130 x 121 slab 1314 -> 1276 us).
 template <int PH, int RE, int RI>
 cudaError_t run_all(const FaceArgs3& a, void (*launched)(cudaStream_t), cudaStream_t s) {
-    const cudaError_t e = cudaMemsetAsync(a.d[0].fix_count, 0, 3 * sizeof(unsigned), s);
-    if (e != cudaSuccess) return e;
     if (!empty(a.d[2])) {
         k_face<PH, RE, RI, false, 2><<<face_grid(a.d[2]), 128, 0, s>>>(a.d[2]);
         launched(s);
@@ -185,16 +192,19 @@ cudaError_t launch_carried(const FaceArgs& a, bool given, void (*launched)(cudaS
 }
 
 cudaError_t launch_all(const FaceArgs* dirs, void (*launched)(cudaStream_t), cudaStream_t s) {
+    // one list for the three passes in the order they run (z, x, y), the counters next to
+    // each other: a third of it for each left one direction alone a rescan of its
+    // whole pass at a third of the faces that it had room for
     FaceArgs3 a;
+    const int order[3] = {1, 2, 0};
     for (int d = 0; d < 3; ++d) {
         a.d[d] = dirs[d];
-        // a third of the list each, the counters next to each other
-        const unsigned cap = dirs[d].fix_cap / 3;
-        a.d[d].fix_count = dirs[0].fix_count + d;
-        a.d[d].fix_list = dirs[0].fix_list + (size_t)d * cap;
-        a.d[d].fix_cap = cap;
+        a.d[d].fix_count = dirs[0].fix_count + order[d];
+        a.d[d].fix_before = order[d];
     }
     if (empty(a.d[0]) && empty(a.d[1]) && empty(a.d[2])) return cudaSuccess;
+    const cudaError_t e = cudaMemsetAsync(dirs[0].fix_count, 0, 3 * sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
     const AstroParams& p = a.d[0].p;
     if (p.physics == ASTRO_SRHD)
         return p.recon == 0 ? run_riemann<ASTRO_SRHD, 0>(a, launched, s)

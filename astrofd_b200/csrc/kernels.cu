@@ -137,8 +137,8 @@ inline bool passive_fluxes(const AstroParams& p) {
     return p.recon == ASTRO_RECON_MUSCL;
 }
 
-// capacity of the float64 fix-up list: a fraction of one face pass; faces
-// beyond it keep their float32 result (counted, never written out of bounds)
+// capacity of the float64 fix-up list: a fraction of one face pass.  Faces beyond it
+// are counted, not listed; their pass is then searched for them
 inline size_t fix_capacity(const AstroGrid& g) {
     const size_t nc = (size_t)g.nx * g.ny * g.nz;
     return nc / 16 + 1024;
