@@ -113,8 +113,9 @@ def _pointwise(fn, comps, gamma=None):
 
 def _rows_of_one_block(comps):
     """The components as one [len(comps), n] view where they are the successive
-    rows of one contiguous float64 CUDA block (`cons_to_prim(*U)`), else None.
-    The copy that stacking makes took a third of a 1 M state conversion."""
+    rows of one contiguous float64 CUDA block (`cons_to_prim(*U)`), else None (a
+    lazily negated view's memory is not its values).  The copy that stacking makes
+    took a third of a 1 M state conversion."""
     import torch
     c0 = comps[0]
     n = c0.numel()
@@ -122,7 +123,7 @@ def _rows_of_one_block(comps):
         return None
     for i, c in enumerate(comps):
         if not (isinstance(c, torch.Tensor) and c.is_cuda and c.dtype == torch.float64
-                and c.shape == c0.shape and c.is_contiguous()
+                and c.shape == c0.shape and c.is_contiguous() and not c.is_neg()
                 and c.untyped_storage().data_ptr() == c0.untyped_storage().data_ptr()
                 and c.storage_offset() == c0.storage_offset() + i * n):
             return None
