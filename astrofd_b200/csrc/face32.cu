@@ -126,9 +126,9 @@ bool empty(const FaceArgs& a) { return a.ext[0] <= 0 || a.ext[1] <= 0 || a.ext[2
 // one direction and its listed faces, for the carried order of passes
 template <int RE, int RI>
 struct OnePass {
-    static cudaError_t run(const FaceArgs& a, bool given, cudaStream_t s) {
+    static cudaError_t run(const FaceArgs& a, bool given, int sms, cudaStream_t s) {
         constexpr int PH = ASTRO_RMHD;
-        const dim3 fgrd(148 * 4), grd = face_grid(a);
+        const dim3 fgrd(sms * 4), grd = face_grid(a);
         const cudaError_t e = cudaMemsetAsync(a.fix_count, 0, sizeof(unsigned), s);
         if (e != cudaSuccess) return e;
         if (given) {
@@ -152,7 +152,7 @@ struct OnePass {
 // launch behind them and one clear precedes them, 5 launches instead of 9
 // (SSPRK3 step of a 75 x 130 x 121 slab 1314 -> 1276 us).
 template <int PH, int RE, int RI>
-cudaError_t run_all(const FaceArgs3& a, void (*launched)(cudaStream_t), cudaStream_t s) {
+cudaError_t run_all(const FaceArgs3& a, int sms, void (*launched)(cudaStream_t), cudaStream_t s) {
     if (!empty(a.d[2])) {
         k_face<PH, RE, RI, false, 2><<<face_grid(a.d[2]), 128, 0, s>>>(a.d[2]);
         launched(s);
@@ -162,36 +162,37 @@ cudaError_t run_all(const FaceArgs3& a, void (*launched)(cudaStream_t), cudaStre
         launched(s);
     }
     if (!empty(a.d[1])) k_face<PH, RE, RI, false, 1><<<face_grid(a.d[1]), 128, 0, s>>>(a.d[1]);
-    k_face_fix3<PH, RE, RI><<<dim3(148, 3), 128, 0, s>>>(a);
+    k_face_fix3<PH, RE, RI><<<dim3(sms, 3), 128, 0, s>>>(a);
     launched(s);
     return cudaGetLastError();
 }
 
 template <int PH, int RE>
-cudaError_t run_riemann(const FaceArgs3& a, void (*launched)(cudaStream_t), cudaStream_t s) {
+cudaError_t run_riemann(const FaceArgs3& a, int sms, void (*launched)(cudaStream_t), cudaStream_t s) {
     const int ri = a.d[0].p.riemann;
     if constexpr (PH == ASTRO_RMHD)
-        if (ri == 2) return run_all<PH, RE, 2>(a, launched, s);
-    return ri == 1 ? run_all<PH, RE, 1>(a, launched, s) : run_all<PH, RE, 0>(a, launched, s);
+        if (ri == 2) return run_all<PH, RE, 2>(a, sms, launched, s);
+    return ri == 1 ? run_all<PH, RE, 1>(a, sms, launched, s) : run_all<PH, RE, 0>(a, sms, launched, s);
 }
 
 }  // namespace
 
-cudaError_t launch_carried(const FaceArgs& a, bool given, void (*launched)(cudaStream_t), cudaStream_t s) {
+cudaError_t launch_carried(const FaceArgs& a, bool given, int sms, void (*launched)(cudaStream_t),
+                           cudaStream_t s) {
     if (empty(a)) return cudaSuccess;
     const int ri = a.p.riemann;
     cudaError_t e;
     if (a.p.recon == ASTRO_RECON_PPM)
-        e = ri == 2 ? OnePass<1, 2>::run(a, given, s)
-                    : (ri == 1 ? OnePass<1, 1>::run(a, given, s) : OnePass<1, 0>::run(a, given, s));
+        e = ri == 2 ? OnePass<1, 2>::run(a, given, sms, s)
+                    : (ri == 1 ? OnePass<1, 1>::run(a, given, sms, s) : OnePass<1, 0>::run(a, given, sms, s));
     else
-        e = ri == 2 ? OnePass<2, 2>::run(a, given, s)
-                    : (ri == 1 ? OnePass<2, 1>::run(a, given, s) : OnePass<2, 0>::run(a, given, s));
+        e = ri == 2 ? OnePass<2, 2>::run(a, given, sms, s)
+                    : (ri == 1 ? OnePass<2, 1>::run(a, given, sms, s) : OnePass<2, 0>::run(a, given, sms, s));
     if (e == cudaSuccess) launched(s);
     return e;
 }
 
-cudaError_t launch_all(const FaceArgs* dirs, void (*launched)(cudaStream_t), cudaStream_t s) {
+cudaError_t launch_all(const FaceArgs* dirs, int sms, void (*launched)(cudaStream_t), cudaStream_t s) {
     // one list for the three passes in the order they run (z, x, y), the counters next to
     // each other: a third of it for each left one direction alone a rescan of its
     // whole pass at a third of the faces that it had room for
@@ -207,12 +208,12 @@ cudaError_t launch_all(const FaceArgs* dirs, void (*launched)(cudaStream_t), cud
     if (e != cudaSuccess) return e;
     const AstroParams& p = a.d[0].p;
     if (p.physics == ASTRO_SRHD)
-        return p.recon == 0 ? run_riemann<ASTRO_SRHD, 0>(a, launched, s)
-                            : (p.recon == 1 ? run_riemann<ASTRO_SRHD, 1>(a, launched, s)
-                                            : run_riemann<ASTRO_SRHD, 2>(a, launched, s));
-    return p.recon == 0 ? run_riemann<ASTRO_RMHD, 0>(a, launched, s)
-                        : (p.recon == 1 ? run_riemann<ASTRO_RMHD, 1>(a, launched, s)
-                                        : run_riemann<ASTRO_RMHD, 2>(a, launched, s));
+        return p.recon == 0 ? run_riemann<ASTRO_SRHD, 0>(a, sms, launched, s)
+                            : (p.recon == 1 ? run_riemann<ASTRO_SRHD, 1>(a, sms, launched, s)
+                                            : run_riemann<ASTRO_SRHD, 2>(a, sms, launched, s));
+    return p.recon == 0 ? run_riemann<ASTRO_RMHD, 0>(a, sms, launched, s)
+                        : (p.recon == 1 ? run_riemann<ASTRO_RMHD, 1>(a, sms, launched, s)
+                                        : run_riemann<ASTRO_RMHD, 2>(a, sms, launched, s));
 }
 
 }  // namespace astro_face32

@@ -950,7 +950,7 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
         a.fix_cap = (unsigned)fix_capacity(g);
         a.speeds_out = (carried && d == 2) ? (void*)(work + L.Sz) : nullptr;
         if (!carried) continue;
-        cudaError_t e = astro_face32::launch_carried(a, false, launched, s);
+        cudaError_t e = astro_face32::launch_carried(a, false, sm_count_cached(), launched, s);
         if (e != cudaSuccess) return e;
         if (d == 0) {
             FaceArgs c = a;
@@ -959,12 +959,12 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
             c.aux = nullptr;
             c.speeds_out = nullptr;
             c.carried = work + L.Sz;
-            e = astro_face32::launch_carried(c, true, launched, s);
+            e = astro_face32::launch_carried(c, true, sm_count_cached(), launched, s);
             if (e != cudaSuccess) return e;
         }
     }
     if (!carried) {
-        const cudaError_t e = astro_face32::launch_all(dirs, launched, s);
+        const cudaError_t e = astro_face32::launch_all(dirs, sm_count_cached(), launched, s);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -1085,7 +1085,7 @@ void launch_ghosts_yz(double* pr, const AstroGrid& g, int ng, cudaStream_t s) {
     const size_t frame = (size_t)g.ny * g.nz - (size_t)(g.ny - 2 * ng) * (g.nz - 2 * ng);
     // x planes over z; past a few waves a thread takes several planes
     const unsigned bx = (unsigned)((frame + 255) / 256);
-    const size_t wave = (size_t)148 * 8 * 4;
+    const size_t wave = (size_t)sm_count_cached() * 8 * 4;
     size_t bz = wave / ((size_t)bx * g.nv) + 1;
     if (bz > (size_t)g.nx) bz = (size_t)g.nx;
     if (bz > 65535) bz = 65535;
@@ -2020,7 +2020,7 @@ int astro_nozzle_left_x(double* pr, const AstroGrid* g, const AstroNozzle* nz,
     // the zero-gradient copy: one variable per blockIdx.y while the cells do not
     // fill the device (256^2 x 3 cells: 13 us, 27 us with a block row per variable,
     // which repeats the profile; 16^2 x 2: 5.2 us, 3.2 us)
-    const size_t spare = (size_t)148 * 2048 / n;
+    const size_t spare = (size_t)sm_count_cached() * 2048 / n;
     const unsigned by = nz->ambient_bc != 1 || spare < 1 ? 1u
                         : (spare < (size_t)g->nv ? (unsigned)spare : var_blocks(g->nv));
     const dim3 grd(grid_for(n, 128), by);
