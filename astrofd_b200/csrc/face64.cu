@@ -18,14 +18,18 @@
 // float64 with IEEE divisions, so overflows end as they do there.
 //
 // The reference's carried x faces (core/rmhd_core.py:1445,1468) differ from the
-// ordinary ones in the wave speeds alone, so both fluxes are formed from one
-// pair of states instead of by two passes.
+// ordinary ones in the wave speeds alone, so both fluxes are formed from one pair of
+// states instead of by two passes (HLLE; "hlld" with carried speeds is Args::exact).
 //
 // Bound: the float64 pipe (about 850 float64 operations per RMHD WENO5 face) at 16
-// warps per SM, 128 registers.  One stage's faces of 134^3 cells, RMHD WENO5 "hlld"
-// with carried x faces: 2204 us as four per-face passes with IEEE divisions, 631 us
-// here; SRHD PPM HLLC 377 us, 220 us.  (RMHD at 3 blocks per SM, which spill nothing,
-// 4 % slower; at 5, 1 %.)
+// warps per SM, 128 registers.  One stage's faces of 134^3 cells, per-face passes with
+// IEEE divisions against this kernel: RMHD WENO5 HLLE with carried x faces 2166 us
+// and 625 us, "hlld" with its own speeds 1802 us and 586 us, MUSCL "hlld" 952 us and
+// 705 us, SRHD PPM HLLC 369 us and 217 us.  (RMHD at 3 blocks per SM, which spill
+// nothing, 4 % slower; at 5, 1 %.)
+//
+// Schemes that amplify last bits (exact_bits in kernels.cu) keep the general per-face
+// evaluation, k_face_general.
 #include "face64.cuh"
 
 #include <stdint.h>
@@ -243,9 +247,10 @@ __device__ __forceinline__ void walk(const Args& a, double* sh, unsigned block) 
                                                  wide);
 }
 
-// Blocks per SM: SRHD 8 (64 registers: 4 blocks at 128 take 723 against 683 us for
-// a 128^3 PPM step's faces, 113 against 89 us for a 64^3 MUSCL one's); RMHD 4 (128
-// registers).
+// Blocks per SM: SRHD 8 (64 registers, which spill 440 to 520 bytes a thread, most of
+// them for the dissipation branch: 4 blocks at 128 take 723 against 683 us for a
+// 128^3 PPM step's faces, 113 against 89 us for a 64^3 MUSCL one's; 5 to 7 were not
+// compared); RMHD 4 (128 registers, at most 70 bytes spilled).
 template <int PHYS, int RECON, int RIEMANN>
 __global__ void __launch_bounds__(T, PHYS == ASTRO_SRHD ? 8 : 4)
     k_face64(const __grid_constant__ Args a) {
@@ -355,8 +360,9 @@ cudaError_t launch(Args a, int sms, void (*launched)(cudaStream_t), cudaStream_t
         // device, up to 16 faces; alone, of the lengths up to 32 the one that needs
         // the fewest turns with whole waves of blocks (128^3 RMHD x faces: 129 as 9
         // segments of 15 are 2 waves, as 19 of 7 they were 5).  Segments of equal
-        // length.  Against 4 waves of walks with z first: ragged 90 x 61 x 103 PPM
-        // faces 174 -> 151 us, Kerr-Schild 72^3 WENO5 163 -> 136 us per stage, SRHD
+        // length.  Against 4 waves of walks with z first, with "hlld" and carried x
+        // faces, which then were this kernel's too: PPM faces of 90 x 61 x 103 cells 174
+        // -> 151 us, WENO5 of 72^3 163 -> 136 us per stage (HLLE now 133 and 132 us); SRHD
         // 128^3 PPM 228 -> 220 us.
         const long per = (e[1 - d] * e[2] + T - 1) / T, faces = e[d] + 1;
         long seg = 1;

@@ -16,8 +16,8 @@
 // The reference's RMHD PPM/WENO x faces use the wave speeds left over from the
 // previous cell's z face (core/rmhd_core.py:1285,1314,1445,1468).  In
 // ASTRO_FLUX_REFERENCE mode those faces get a second flux with the carried
-// speeds, read from the z-face speed buffer (float32: a second pass, k_face<GIVEN>;
-// float64: from the same states in the same pass); in ASTRO_FLUX_CONSERVATIVE mode
+// speeds, read from the z-face speed buffer (a second pass; float64 HLLE: from the same
+// states in the same pass); in ASTRO_FLUX_CONSERVATIVE mode
 // every face uses its own speeds, so each face flux enters both neighbours and
 // the scheme conserves D, S, tau exactly.
 #include <cuda_runtime.h>

@@ -881,7 +881,10 @@ AHD double r_f_of_Z(const Phys<double>& P, double Z, double D, double tau, doubl
 
 // f(Z) with the divisions regrouped (FAST, r_f_df_of_Z: a third of the float64
 // operations, a dependency chain half as long) or in the reference's operation
-// order; equal to rounding.  The reference's order is kept for PPM blocks, whose
+// order; equal to rounding (2e5 strongly magnetised states with several roots: 2.4e-3
+// and 2.3e-3 of them further than 1e-10 from the reference's result, 2.2e-3 after one
+// ulp of tau).  The reference's order is kept where its rounding would show (c2p_fast in
+// kernels.cu): for schemes that amplify last bits, the mixed path, and PPM, whose
 // flattening test compares neighbouring cells: in the cells outside the updated
 // range, which every stage converts to and fro, pressures that began equal differ
 // by the conversion's rounding alone, and its sign then switches a face value by
