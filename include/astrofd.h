@@ -12,7 +12,8 @@
  *     default stream.  All entry points are stream-ordered and asynchronous
  *     unless stated otherwise; none synchronises the device.
  *   - Scratch memory is caller-owned: query its size with the matching
- *     *_workspace_bytes() call and pass a device buffer of at least that size.
+ *     *_workspace_bytes() call and pass a device buffer of at least that size,
+ *     aligned for float64 as the blocks are (the fused stages: 16 bytes).
  *   - Return value: 0 on success, a negative ASTRO_E* code on failure
  *     (astro_error_string() describes it).  Numerical failures inside kernels
  *     (con2prim falling back, iteration caps) never trap: they are counted in
@@ -285,7 +286,11 @@ int astro_outflow_yz(double* pr, const AstroGrid* g, int ng, void* stream);
  * Array forms of prim_to_cons / cons_to_prim (core/srhd_core.py:47,62) and
  * prim_to_cons_rmhd / cons_to_prim_rmhd (core/rmhd_core.py:138,249).
  * Arrays are (nm, count) float64.  For these and the batch calls below a
- * count of 0 does nothing and returns ASTRO_OK, with null arrays allowed. */
+ * count of 0 does nothing and returns ASTRO_OK, with null arrays allowed.
+ * RMHD astro_c2p rounds as the steps of the same parameters do: in the
+ * reference's order of operations for PPM, the mixed path and schemes that
+ * amplify last bits, with regrouped divisions otherwise (the same equation
+ * and tolerance, about half the time). */
 int astro_p2c(const AstroParams* p, const double* prim, double* cons, int64_t count,
               void* stream);
 int astro_c2p(const AstroParams* p, const double* cons, double* prim, int64_t count,
