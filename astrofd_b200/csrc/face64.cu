@@ -107,6 +107,8 @@ template <int RECON>
 __device__ __forceinline__ void recon_cell(const double* q, int lim, double& lo, double& hi, bool& wide) {
     if constexpr (RECON == ASTRO_RECON_MUSCL) {
         const double s = limiter(lim, fd(q[2] - q[1]), fd(q[3] - q[2])).v;
+        // van Leer's denominator beyond the reciprocal's range
+        wide |= lim == ASTRO_LIM_VANLEER && beyond(fd(q[3] - q[1]));
         lo = q[2] - 0.5 * s;
         hi = q[2] + 0.5 * s;
     } else if constexpr (RECON == ASTRO_RECON_PPM) {
@@ -196,7 +198,7 @@ __device__ __forceinline__ void cell_and_face(const Args& a, double* sh, int i, 
             }
             fd G[9];
             r_riemann<RIEMANN, OVR>(P, 0, qL, qR, UL, UR, FL, FR, fd(cL), fd(cR), G);
-            bool okc = !wide;
+            bool okc = !wide && isfinite(sL.v);
 #pragma unroll
             for (int v = 0; v < 9; ++v) {
                 okc &= isfinite(G[v].v);

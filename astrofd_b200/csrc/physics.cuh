@@ -118,7 +118,8 @@ AHD double rcp_nr(double x) {
 // three or five of the float64 pipe, without the range tests and the slow branch of
 // an IEEE division.  For normal arguments: zero, infinity, subnormals and, under the
 // root, negative values give a result that is not finite, which sends the face to the
-// general evaluation.  The reciprocal of a value beyond 2^1022 (a subnormal) is zero.
+// general evaluation.  The reciprocal of a value beyond 2^1022 (a subnormal) is zero,
+// which beyond() keeps from the callers.
 template <> AHD fd rcp_(fd x) {
 #ifdef __CUDA_ARCH__
     double r;
@@ -137,6 +138,16 @@ template <> AHD fd rsq_(fd x) {
     return fd(fma(r * e, fma(0.375, e, 0.5), r));
 #else
     return fd(1.0 / sqrt(x.v));
+#endif
+}
+// |x| >= 2^900, infinite or NaN, by its exponent: a bound on a face's conserved density
+// and energy that leaves its denominators, a contact speed of 1e12 times them
+// included, below 2^1022
+AHD bool beyond(fd x) {
+#ifdef __CUDA_ARCH__
+    return (__double2hiint(x.v) & 0x7fffffff) >= 0x78300000;
+#else
+    return !(x.v < 0x1p900 && x.v > -0x1p900);
 #endif
 }
 // sqrt(x) for x >= 0 (what its callers clamp to): x / sqrt(x) with the argument kept
@@ -335,6 +346,16 @@ template <typename R> AHD void eig_speeds(R vn, R cs, R& lm, R& lp) {
     lm = m; lp = p;
 }
 
+// The lower speed of an fd face: NaN where a state is beyond the reciprocals' range, also
+// where the other side's flux alone is taken, so that the face goes to the general
+// evaluation.  A NaN speed of the left state stays in it (rmin takes its second argument
+// then), one of the right state in the upper speed's rmax(left, right); a finite state
+// shows in its conserved density and energy, which bound every denominator.
+AHD fd fd_speed(fd lmL, fd lmR, const fd* UL, const fd* UR) {
+    const bool out = beyond(UL[0]) | beyond(UL[4]) | beyond(UR[0]) | beyond(UR[4]);
+    return out ? fd(NAN) : rmin(lmR, lmL);
+}
+
 // ----------------------------------------------------------------- SRHD ---
 template <typename R> AHD void s_p2c(const Phys<R>& P, const R* q, R* U) {
     const R gamma = P.srhd_gamma;
@@ -469,7 +490,11 @@ AHD void s_face(const Phys<R>& P, int n, R* qL, R* qR, R* F, R& sL, R& sR, int n
     R csL = s_sound_speed(P, qL[0], qL[4]), csR = s_sound_speed(P, qR[0], qR[4]);
     eig_speeds(qL[1 + n], csL, lmL, lpL);
     eig_speeds(qR[1 + n], csR, lmR, lpR);
-    sL = kRecip<R> && sizeof(R) == 8 ? rmin(lmR, lmL) : rmin(lmL, lmR);  // fd: see r_face_states
+    if constexpr (kRecip<R> && sizeof(R) == 8) {
+        sL = fd_speed(lmL, lmR, UL, UR);
+    } else {
+        sL = rmin(lmL, lmR);
+    }
     sR = rmax(lpL, lpR);
     if (RIEMANN == ASTRO_RIEMANN_HLLC)
         hllc5(n, UL, UR, FL, FR, sL, sR, qL[4], qR[4], qL[1 + n], qR[1 + n], F);
@@ -764,10 +789,7 @@ AHD void r_face_states(const Phys<fd>& P, int n, fd* qL, fd* qR, fd* UL, fd* UR,
     r_flux_u(P, n, qR, UR, FR, BBR, vbR);
     eig_speeds(qL[1 + n], r_fast_speed_from(P, qL[4], rhL, b2L), lmL, lpL);
     eig_speeds(qR[1 + n], r_fast_speed_from(P, qR[4], rhR, b2R), lmR, lpR);
-    // a NaN of the left state stays in sL (rmin takes its second argument then) and one of
-    // the right state in sR: a state beyond the reciprocals' range sends the face to the
-    // general evaluation even where the other side's flux alone is taken
-    sL = rmin(lmR, lmL);
+    sL = fd_speed(lmL, lmR, UL, UR);
     sR = rmax(lpL, lpR);
 }
 
