@@ -97,10 +97,10 @@ def test_the_restatement_is_the_oracles_scheme(seed):
 @pytest.mark.gpu
 @pytest.mark.parametrize("seed", [1, 2, 3])
 def test_face_rounding(seed):
-    """The reference's own form, weights over their sum times polynomials, rounds each
-    face value by about one half ulp rms (1.0 measured); the differences from the middle
-    polynomial, weighted, by 0.5 to 0.6.  So the right-hand side's error is below the
-    oracle's; 0.8 of it allows for the rest of the face."""
+    """The reference's own form, six divisions for the weights of a face, rounds a face
+    value by about one half ulp rms, most of it the weights' (1.0 measured, without
+    them 0.5 to 0.7).  So the right-hand side's error is below the oracle's; 0.8 of it allows
+    for the rest of the face."""
     import torch
     from astrofd_b200.core import srhd_core
     pr = _beam(seed)
@@ -110,3 +110,27 @@ def test_face_rounding(seed):
     ref = O.rhs(O.params_from_config("srhd", CFG), pr, *D)
     e, r = _error(got, exact), _error(ref, exact)
     assert np.all(e <= 0.8 * r), (e, r)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("jump", [1e6, 1e12, 1e20])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_a_jump_stays_behind_its_stencils(jump, axis):
+    """Two cells from a plane of 1e6 to 1e20 times the density every face value comes from
+    stencils that leave it out: the other stencils' weights are below (1e-12 / jump^2)^2
+    there, and no rounding of the weights may bring their polynomials back."""
+    import torch
+    from astrofd_b200.core import srhd_core
+    pr = _beam(4)
+    at = [slice(None)] * 3
+    at[axis] = 10
+    pr[(0,) + tuple(at)] *= jump
+    srhd_core.configure(CFG)
+    got = srhd_core.compute_rhs_weno(torch.from_numpy(pr).cuda(), *pr.shape[1:], *D).cpu().numpy()
+    ref = O.rhs(O.params_from_config("srhd", CFG), pr, *D)
+    for side in (slice(3, 9), slice(12, pr.shape[1 + axis] - 3)):
+        at[axis] = side
+        for v in range(5):
+            x, y = got[(v,) + tuple(at)], ref[(v,) + tuple(at)]
+            # the bar of the fixture comparison: FMA and division rounding
+            assert np.abs(x - y).max() <= 1e-11 * np.abs(y).max()
