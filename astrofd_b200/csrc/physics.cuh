@@ -806,7 +806,7 @@ struct C2PCount {
 // g = gamma / (gamma - 1), and E - D <= p0 / (gamma - 1) unless p0 was clamped
 // to P_MAX, so for every p >= p0
 //   -f(p) >= D (W - 1) + g p (W^2 - 1) + (p - p0) / (gamma - 1).
-// A first step upwards that is not yet within the tolerance is therefore
+// A first step upwards that is clear of the tolerance and of rounding is therefore
 // followed by steps upwards only, none of them smaller (gamma < 2): the
 // iteration runs away from its root to P_MAX, never converges, and the result
 // is p0.  (From a p0 clamped to P_MAX such a step returns to P_MAX, 60 times.)
@@ -841,9 +841,12 @@ AHD void s_c2p(const Phys<double>& P, const double* U, double* q) {
         if (pn < SM) pn = SM;
         if (pn > P.p_max) pn = P.p_max;
         if (fabs(dp) < 1e-12 * rmax(1.0, pn)) { p = pn; ok = true; break; }
-        // runs away (see above); D > 2e-12 W keeps rho off its floor for this
-        // and every larger p (W falls with p)
-        if (it == 0 && dp > 0.0 && D > 2.0 * SM * W && gamma > 1.0 && gamma < 2.0) break;
+        // runs away (see above), by more than the tolerance and f's rounding of a few
+        // ulp of E, which later steps could converge by; D > 2e-12 W keeps rho off its
+        // floor for this and every larger p (W falls with p)
+        if (it == 0 && -f > 1.1e-12 * rmax(1.0, pn) + 1e-14 * E && D > 2.0 * SM * W && gamma > 1.0 &&
+            gamma < 2.0)
+            break;
         p = pn;
     }
     if (!ok) {
