@@ -26,12 +26,11 @@ struct FaceArgs {
     int ndiss;           // SRHD Israel-Stewart blocks: dissipation fluxes per face
     AstroParams p;
     // float32 passes: faces whose float32 result is not finite are listed here
-    // and recomputed in float64 by k_face_fix
+    // and recomputed in float64 by k_face_fix.  The two words in front of the count
+    // are those of the passes whose faces stand before this one's in the list, or zero
     unsigned* fix_count;
     unsigned* fix_list;
     unsigned fix_cap;
-    int fix_before;      // earlier passes whose faces stand before this one's in the
-                         // list; their counts are in front of fix_count
 };
 
 // One face: reconstruct, floor, p2c, flux, speeds, Riemann in arithmetic R,

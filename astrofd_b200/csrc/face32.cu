@@ -11,9 +11,7 @@ namespace {
 // first place of this pass in the list of faces to recompute: behind the faces that the
 // passes before it (complete by now: one stream) have counted
 __device__ __forceinline__ size_t fix_base(const FaceArgs& a) {
-    size_t n = 0;
-    for (int q = 1; q <= a.fix_before; ++q) n += a.fix_count[-q];
-    return n;
+    return (size_t)a.fix_count[-1] + a.fix_count[-2];
 }
 
 // float32 face pass of one direction (the float64 passes are face64.cu's)
@@ -129,7 +127,7 @@ struct OnePass {
     static cudaError_t run(const FaceArgs& a, bool given, int sms, cudaStream_t s) {
         constexpr int PH = ASTRO_RMHD;
         const dim3 fgrd(sms * 4), grd = face_grid(a);
-        const cudaError_t e = cudaMemsetAsync(a.fix_count, 0, sizeof(unsigned), s);
+        const cudaError_t e = cudaMemsetAsync(a.fix_count - 2, 0, 3 * sizeof(unsigned), s);
         if (e != cudaSuccess) return e;
         if (given) {
             k_face<PH, RE, RI, true, 0><<<grd, 128, 0, s>>>(a);
@@ -201,10 +199,9 @@ cudaError_t launch_all(const FaceArgs* dirs, int sms, void (*launched)(cudaStrea
     for (int d = 0; d < 3; ++d) {
         a.d[d] = dirs[d];
         a.d[d].fix_count = dirs[0].fix_count + order[d];
-        a.d[d].fix_before = order[d];
     }
     if (empty(a.d[0]) && empty(a.d[1]) && empty(a.d[2])) return cudaSuccess;
-    const cudaError_t e = cudaMemsetAsync(dirs[0].fix_count, 0, 3 * sizeof(unsigned), s);
+    const cudaError_t e = cudaMemsetAsync(dirs[0].fix_count - 2, 0, 5 * sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
     const AstroParams& p = a.d[0].p;
     if (p.physics == ASTRO_SRHD)

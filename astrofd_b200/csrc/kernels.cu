@@ -945,7 +945,7 @@ cudaError_t face_passes(const AstroParams& p, const AstroGrid& g, const Bounds& 
         }
         a.F = work + L.F[d];
         a.aux = passive_fluxes(p) ? (void*)(work + L.aux[d]) : nullptr;
-        a.fix_count = (unsigned*)(work + L.fix);
+        a.fix_count = (unsigned*)(work + L.fix) + 2;  // see FaceArgs
         a.fix_list = (unsigned*)(work + L.fix + 256);
         a.fix_cap = (unsigned)fix_capacity(g);
         a.speeds_out = (carried && d == 2) ? (void*)(work + L.Sz) : nullptr;

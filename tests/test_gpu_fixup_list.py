@@ -51,8 +51,9 @@ def test_one_direction_may_fill_the_list():
     # the workspace: three flux blocks of 9 float32 rows, then the counters, then the list
     off = 3 * ((9 * nc * 4 + 255) // 256 * 256)
     words = w[off:off + 256 + 4 * cap].cpu().numpy().view(np.uint32)
-    listed, lst = int(words[0]), words[64:]
-    assert words[1:3].tolist() == [0, 0]
+    # two zero words, then the counts of z, x and y
+    listed, lst = int(words[2]), words[64:]
+    assert words[[0, 1, 3, 4]].tolist() == [0, 0, 0, 0]
     assert cap // 3 < listed <= cap
     e = (N[0], N[1], N[2] + 1)  # z faces
     c = sorted(k + o - NG for k in PLANES for o in (0, 1))
