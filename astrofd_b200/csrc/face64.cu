@@ -23,9 +23,9 @@
 //
 // Bound: the float64 pipe (about 850 float64 operations per RMHD WENO5 face) at 16
 // warps per SM, 128 registers.  One stage's faces of 134^3 cells, per-face passes with
-// IEEE divisions against this kernel: RMHD WENO5 HLLE with carried x faces 2166 us
-// and 625 us, "hlld" with its own speeds 1802 us and 586 us, MUSCL "hlld" 952 us and
-// 705 us, SRHD PPM HLLC 369 us and 217 us.  (RMHD at 3 blocks per SM, which spill
+// IEEE divisions against this kernel: RMHD WENO5 HLLE with carried x faces 2175 us
+// and 597 us, "hlld" with its own speeds 1819 us and 558 us, MUSCL "hlld" 953 us and
+// 722 us, SRHD PPM HLLC 370 us and 220 us.  (RMHD at 3 blocks per SM, which spill
 // nothing, 4 % slower; at 5, 1 %.)
 //
 // Schemes that amplify last bits (exact_bits in kernels.cu) keep the general per-face
@@ -72,7 +72,7 @@ __device__ __noinline__ void general_face(const Args& a, int i, int j, int k) {
 // back with the last bit of 1.  L2 distance of right-hand sides of a 40 x 37 x 45 jet from
 // 80-bit arithmetic, x and y momentum: 1.9e-14 and 1.5e-14; without that factor 3.7e-14
 // and 3.3e-14; with the reference's six divisions 2.7e-14 and 1.7e-14.  It costs no time
-// (128^3 RMHD HLLE 601 us per stage with it, 604 without; SRHD HLLC 321 and 305).
+// (128^3 RMHD HLLE 601 us per stage with it, 604 without; SRHD HLLC 318 and 303).
 __device__ __forceinline__ void weno5_cell(const double* q, double& lo, double& hi, bool& wide) {
     const double a = q[0], b = q[1], c = q[2], d = q[3], e = q[4];
     const double d0 = b - a, d1 = c - b, d2 = d - c, d3 = e - d;
@@ -368,7 +368,7 @@ cudaError_t launch(Args a, int sms, void (*launched)(cudaStream_t), cudaStream_t
         // segments of 15 are 2 waves, as 19 of 7 they were 5).  Segments of equal
         // length.  Against 4 waves of walks with z first, with "hlld" and carried x
         // faces, which then were this kernel's too: PPM faces of 90 x 61 x 103 cells 174
-        // -> 151 us, WENO5 of 72^3 163 -> 136 us per stage (HLLE now 133 and 132 us); SRHD
+        // -> 151 us, WENO5 of 72^3 163 -> 136 us per stage (HLLE now 134 and 133 us); SRHD
         // 128^3 PPM 228 -> 220 us.
         const long per = (e[1 - d] * e[2] + T - 1) / T, faces = e[d] + 1;
         long seg = 1;

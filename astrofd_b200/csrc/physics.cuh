@@ -350,11 +350,8 @@ template <typename R> AHD void eig_speeds(R vn, R cs, R& lm, R& lp) {
 // where the other side's flux alone is taken, so that the face goes to the general
 // evaluation.  A NaN speed of the left state stays in it (rmin takes its second argument
 // then), one of the right state in the upper speed's rmax(left, right); a finite state
-// shows in its conserved density and energy, which bound every denominator.
-AHD fd fd_speed(fd lmL, fd lmR, const fd* UL, const fd* UR) {
-    const bool out = beyond(UL[0]) | beyond(UL[4]) | beyond(UR[0]) | beyond(UR[4]);
-    return out ? fd(NAN) : rmin(lmR, lmL);
-}
+// shows in its conserved density and energy, which bound every denominator (out).
+AHD fd fd_speed(fd lmL, fd lmR, bool out) { return out ? fd(NAN) : rmin(lmR, lmL); }
 
 // ----------------------------------------------------------------- SRHD ---
 template <typename R> AHD void s_p2c(const Phys<R>& P, const R* q, R* U) {
@@ -491,7 +488,8 @@ AHD void s_face(const Phys<R>& P, int n, R* qL, R* qR, R* F, R& sL, R& sR, int n
     eig_speeds(qL[1 + n], csL, lmL, lpL);
     eig_speeds(qR[1 + n], csR, lmR, lpR);
     if constexpr (kRecip<R> && sizeof(R) == 8) {
-        sL = fd_speed(lmL, lmR, UL, UR);
+        // w = rho + g p <= D + g P_MAX: the densities are enough
+        sL = fd_speed(lmL, lmR, beyond(UL[0]) | beyond(UR[0]) | beyond(P.p_max));
     } else {
         sL = rmin(lmL, lmR);
     }
@@ -789,7 +787,7 @@ AHD void r_face_states(const Phys<fd>& P, int n, fd* qL, fd* qR, fd* UL, fd* UR,
     r_flux_u(P, n, qR, UR, FR, BBR, vbR);
     eig_speeds(qL[1 + n], r_fast_speed_from(P, qL[4], rhL, b2L), lmL, lpL);
     eig_speeds(qR[1 + n], r_fast_speed_from(P, qR[4], rhR, b2R), lmR, lpR);
-    sL = fd_speed(lmL, lmR, UL, UR);
+    sL = fd_speed(lmL, lmR, beyond(UL[0]) | beyond(UL[4]) | beyond(UR[0]) | beyond(UR[4]));
     sR = rmax(lpL, lpR);
 }
 
