@@ -233,7 +233,6 @@ struct UpdArgs {
     double idd[3], idd2[3];
     int stage, nstages, rhs_only;
     int defer_c2p;       // learned con2prim: write U every stage, primitives later
-    int exact;           // flux differences divided to the last bit
     int frame_only;      // only the cells outside the updated range (the fused
                          // stage kernel updates the others)
     AstroParams p;
@@ -338,43 +337,33 @@ __global__ void __launch_bounds__(kUpdateBlock, PASSIVE ? 1 : 8) k_update(UpdArg
         if (in) {
             // by 1/dx from the host: 27 float64 divisions per cell were most of
             // the update's instructions (float64 RMHD, 78^3 cells: 72 us with
-            // them, 44 us without)
+            // them, 44 us without).  Float64 fluxes: corrected to the quotients'
+            // last bit, as divisions where one is not finite (128^3 RMHD HLLE update
+            // 278 us, 332 us with the bare products; 72^3 68 and 59 us)
             const double i0 = a.idd[0], i1 = a.idd[1], i2 = a.idd[2];
-            bool divide = false;
-            if constexpr (sizeof(RF) == 8 && C2P != kC2PFast) {
-                if (a.exact) {
-                    // the quotients to the last bit, as divisions where one
-                    // is not finite
-                    bool ok = true;
+            bool ok = true;
 #pragma unroll
-                    for (int v = 0; v < NM; ++v) {
-                        double r = 0.0;
-                        r -= quot_(flux(0, v, 1) - flux(0, v, 0), a.dd[0], i0);
-                        r -= quot_(flux(1, v, 1) - flux(1, v, 0), a.dd[1], i1);
-                        r -= quot_(flux(2, v, 1) - flux(2, v, 0), a.dd[2], i2);
-                        rhs[v] = r;
-                        ok &= isfinite(r);
-                    }
-                    if (!ok) {
-#pragma unroll
-                        for (int v = 0; v < NM; ++v) {
-                            double r = 0.0;
-                            r -= (flux(0, v, 1) - flux(0, v, 0)) / a.dd[0];
-                            r -= (flux(1, v, 1) - flux(1, v, 0)) / a.dd[1];
-                            r -= (flux(2, v, 1) - flux(2, v, 0)) / a.dd[2];
-                            rhs[v] = r;
-                        }
-                    }
-                    divide = true;
-                }
-            }
-            if (!divide) {
-#pragma unroll
-                for (int v = 0; v < NM; ++v) {
-                    double r = 0.0;
+            for (int v = 0; v < NM; ++v) {
+                double r = 0.0;
+                if constexpr (sizeof(RF) == 8) {
+                    r -= quot_(flux(0, v, 1) - flux(0, v, 0), a.dd[0], i0);
+                    r -= quot_(flux(1, v, 1) - flux(1, v, 0), a.dd[1], i1);
+                    r -= quot_(flux(2, v, 1) - flux(2, v, 0), a.dd[2], i2);
+                    ok &= isfinite(r);
+                } else {
                     r -= (flux(0, v, 1) - flux(0, v, 0)) * i0;
                     r -= (flux(1, v, 1) - flux(1, v, 0)) * i1;
                     r -= (flux(2, v, 1) - flux(2, v, 0)) * i2;
+                }
+                rhs[v] = r;
+            }
+            if (!ok) {
+#pragma unroll
+                for (int v = 0; v < NM; ++v) {
+                    double r = 0.0;
+                    r -= (flux(0, v, 1) - flux(0, v, 0)) / a.dd[0];
+                    r -= (flux(1, v, 1) - flux(1, v, 0)) / a.dd[1];
+                    r -= (flux(2, v, 1) - flux(2, v, 0)) / a.dd[2];
                     rhs[v] = r;
                 }
             }
@@ -839,8 +828,8 @@ void launch_update_t(const UpdArgs& a, dim3 grd, cudaStream_t s) {
     }
 }
 
-// Schemes that keep the general evaluation's last bit in every part (faces, update,
-// con2prim), in steps, fixed-metric steps and right-hand sides: float64 "hlld" with the
+// Schemes that keep the general evaluation's last bit in every part (faces and
+// con2prim; the update's quotients are exact for all), in steps, fixed-metric steps and right-hand sides: float64 "hlld" with the
 // carried x-face speeds, and "hlld_full".  A contact speed beside speeds that are not
 // its face's divides by s - sM with no lower bound, so a last bit anywhere in a
 // stage comes out of the next one up to 1e9 times larger.  Jets of W = 7 at 128^3, the
@@ -877,7 +866,7 @@ cudaError_t launch_update(const UpdArgs& a, cudaStream_t s) {
         if (a.defer_c2p) launch_update_t<ASTRO_SRHD, kC2PDefer>(a, grd, s);
         else launch_update_t<ASTRO_SRHD, kC2PFast>(a, grd, s);
     } else if (a.defer_c2p) launch_update_t<ASTRO_RMHD, kC2PDefer>(a, grd, s);
-    else if (a.rhs_only ? !a.exact : c2p_fast(a.p)) launch_update_t<ASTRO_RMHD, kC2PFast>(a, grd, s);
+    else if (a.rhs_only || c2p_fast(a.p)) launch_update_t<ASTRO_RMHD, kC2PFast>(a, grd, s);
     else launch_update_t<ASTRO_RMHD, kC2PReference>(a, grd, s);
     mark(1, s);
     return cudaGetLastError();
@@ -986,7 +975,6 @@ UpdArgs update_args(const AstroParams& p, const AstroGrid& g, const Bounds& b, c
         u.idd[d] = 1.0 / u.dd[d];
         u.idd2[d] = 1.0 / (u.dd[d] * u.dd[d] + 1e-12);
     }
-    u.exact = exact_bits(p) ? 1 : 0;
     u.p = p;
     return u;
 }

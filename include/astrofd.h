@@ -237,8 +237,7 @@ int astro_debug_set_tile_poll_limit(long long polls);
 int astro_debug_rcp_f64(const double* x, double* y, int64_t n, void* stream);
 /* Test hook, no counterpart in the reference: what stands in for IEEE operations
  * elsewhere, y[i] = 1 / x[i] (op 0), 1 / sqrt(x[i]) (1) and sqrt(x[i]) (2) of the
- * float64 faces, x[i] / d (3) of the updates that keep a quotient's last bit.  Device
- * arrays. */
+ * float64 faces, x[i] / d (3) of the float64 updates.  Device arrays. */
 int astro_debug_math_f64(int op, const double* x, double d, double* y, int64_t n, void* stream);
 /* Test hook, no counterpart in the reference: Newton polish steps the
  * learned con2prim of astro_step / astro_step_stage / astro_step_gr allows
